@@ -1540,7 +1540,8 @@ GBPT_API int gbpt_trace_primary(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera
         ctx->hits_cap = n;
     }
     rc = trace_primary(it->second, *camera, width, height, instance_mask, ctx->d_hits,
-                       reinterpret_cast<uint32_t*>(ctx->d_misc + 2), ctx->stream);
+                       reinterpret_cast<uint32_t*>(ctx->d_misc + 2), ctx->stream,
+                       sched_of(ctx->tuning));
     if (rc) {
         set_error("gbpt_trace_primary: launch failed");
         return rc;
@@ -1567,7 +1568,8 @@ GBPT_API int gbpt_gbuffer(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* came
         return GBPT_ERR_NOT_FOUND;
     }
     rc = gbuffer(it->second, *camera, width, height, instance_mask, out_device,
-                 reinterpret_cast<uint32_t*>(ctx->d_misc + 2), ctx->stream);
+                 reinterpret_cast<uint32_t*>(ctx->d_misc + 2), ctx->stream,
+                 sched_of(ctx->tuning));
     if (rc) set_error("gbpt_gbuffer: launch failed");
     return rc;
 }

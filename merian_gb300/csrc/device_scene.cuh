@@ -285,15 +285,15 @@ GBPT_DI float3 xform_vector(float4 r0, float4 r1, float4 r2, float3 v) {
 }
 
 // ---- traversal state and loop ------------------------------------------------------------------
-// One loop serves the per-thread queries (trace_ray) and the persistent warps (trace_persistent).
-// In the persistent form a lane postpones its pending triangle tests (pushes the triangle group
-// onto its stack) when fewer than `postpone_lanes` lanes of the warp have triangles to test, so
-// node steps and triangle steps stay in lockstep across the warp, and the warp leaves the loop to
-// refill idle lanes once fewer than `refill_lanes` lanes are busy (both launch arguments). Two-level scenes: a top-level leaf is an
-// instance; entering it pushes what is left of the top level, transforms the ray to object space
-// (t is unchanged: the direction is not renormalised) and continues from the BLAS root; when the
-// stack drops back to the entry depth the world ray is restored. The closest hit and the tie rule
-// (equal t: smallest geometry, primitive, instance) do not depend on the visit order.
+// One loop serves every query (trace_persistent): a lane postpones its pending triangle tests
+// (pushes the triangle group onto its stack) when fewer than `postpone_lanes` lanes of the warp
+// have triangles to test, so node steps and triangle steps stay in lockstep across the warp, and
+// the warp leaves the loop to refill idle lanes once fewer than `refill_lanes` lanes are busy
+// (both launch arguments). Two-level scenes: a top-level leaf is an instance; entering it pushes
+// what is left of the top level, transforms the ray to object space (t is unchanged: the
+// direction is not renormalised) and continues from the BLAS root; when the stack drops back to
+// the entry depth the world ray is restored. The closest hit and the tie rule (equal t: smallest
+// geometry, primitive, instance) do not depend on the visit order.
 
 
 struct TraceState {
@@ -507,14 +507,14 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
 }
 
 // Runs the traversal of the ray in s until it is finished (returns true; result in s.best, geom
-// = kNoInst on a miss; with ANY the first hit found) or, with WARP, until the warp should refill
-// its idle lanes (returns false; s keeps the state). `st(i)` is stack entry i. A stack overflow
-// raises *err and finishes the ray with what it found.
+// = kNoInst on a miss; with ANY the first hit found) or until the warp should refill its idle
+// lanes (returns false; s keeps the state). `st(i)` is stack entry i. A stack overflow raises *err
+// and finishes the ray with what it found.
 // `alpha(geom, prim, u, v)` decides the candidate hits of non-opaque triangles (true: skip).
-template <bool ANY, bool COUNT, bool TWO_LEVEL, bool WARP, class StackRef, class Alpha>
+template <bool ANY, bool COUNT, bool TWO_LEVEL, class StackRef, class Alpha>
 GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32_t* err,
-                        bool pool_empty, const Alpha& alpha, int refill_lanes = 0,
-                        int postpone_lanes = 0) {
+                        bool pool_empty, const Alpha& alpha, int refill_lanes,
+                        int postpone_lanes) {
     while (true) {
         if (s.ngroup.y > 0x00FFFFFFu) {
             const uint32_t hits = s.ngroup.y;
@@ -551,7 +551,7 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
         bool done_any = false;
         // only groups followed by node work are postponed (a group popped back is tested), and
         // never those of a first-hit query, which any of its triangles may end
-        const bool may_postpone = WARP && !ANY && s.ngroup.y > 0x00FFFFFFu;
+        const bool may_postpone = !ANY && s.ngroup.y > 0x00FFFFFFu;
         while (s.tgroup.y != 0u) {
             if (may_postpone && s.sp() < kStackSize && __popc(__activemask()) < postpone_lanes) {
                 st(s.sp()) = s.tgroup;
@@ -630,7 +630,7 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
             }
         }
         if (done) break;
-        if (WARP && !pool_empty && __popc(__activemask()) < refill_lanes) return false;
+        if (!pool_empty && __popc(__activemask()) < refill_lanes) return false;
     }
 #if GBPT_DEFER_UV
     if (s.best.geom != kNoInst) {
@@ -639,27 +639,6 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
     }
 #endif
     return true;
-}
-
-// Closest hit (ANY = false) or first hit (ANY = true) of one ray, per thread. Sets *err when the
-// traversal stack would overflow (the builder bounds the depth, so this does not happen for
-// trees it accepted).
-template <bool ANY, bool COUNT>
-__device__ __forceinline__ Hit trace_ray(const DevScene& sc, float3 o, float3 d, float tmin,
-                                         float tmax, uint32_t ray_mask, TraceCounters* ctr,
-                                         uint32_t* err) {
-    TraceState s;
-    s.nodes = sc.nodes;
-    s.tris_base = sc.tris;
-    s.tri_stride = sc.tri_stride;
-    s.insts = sc.n_inst ? sc.inst : nullptr;
-    s.mask = ray_mask;
-    trace_init(s, o, d, tmin, tmax);
-    uint2 stack[kStackSize];
-    trace_loop<ANY, COUNT, true, false>(
-        s, [&](int i) -> uint2& { return stack[i]; }, ctr, err, true,
-        [&](uint32_t g, uint32_t p, float u, float v) { return alpha_discard(sc, g, p, u, v); });
-    return s.best;
 }
 
 // Runs the traversal of every ray i < n with persistent warps that pull ray indices from *fetch
@@ -704,7 +683,7 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
         const auto ray_alpha = [&](uint32_t g, uint32_t p, float u, float v) {
             return alpha(ray, g, p, u, v);
         };
-        if (trace_loop<ANY, COUNT, TWO_LEVEL, true>(s, st_ref, ctr, err, pool_empty, ray_alpha,
+        if (trace_loop<ANY, COUNT, TWO_LEVEL>(s, st_ref, ctr, err, pool_empty, ray_alpha,
                                                     refill_lanes, postpone_lanes)) {
             store(ray, s.best);
             active = false;

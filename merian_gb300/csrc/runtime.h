@@ -246,9 +246,11 @@ int trace_rays(const SceneGPU& scene, const gbpt_ray* rays, uint32_t n, uint32_t
                gbpt_hit* hits, unsigned long long* counters_device, cudaStream_t stream,
                const TraceSched& sched = TraceSched{});
 int trace_primary(const SceneGPU& scene, const gbpt_camera& cam, uint32_t w, uint32_t h,
-                  uint32_t mask, gbpt_hit* hits_device, uint32_t* err_device, cudaStream_t stream);
+                  uint32_t mask, gbpt_hit* hits_device, uint32_t* err_device, cudaStream_t stream,
+                  const TraceSched& sched = TraceSched{});
 int gbuffer(const SceneGPU& scene, const gbpt_camera& cam, uint32_t w, uint32_t h, uint32_t mask,
-            gbpt_gbuffer_texel* out_device, uint32_t* err_device, cudaStream_t stream);
+            gbpt_gbuffer_texel* out_device, uint32_t* err_device, cudaStream_t stream,
+            const TraceSched& sched = TraceSched{});
 int work_reserve(Work& work, uint64_t paths, uint64_t pixels);
 void work_free(Work& work);
 

@@ -5,8 +5,9 @@
 // camera, spp, path length, estimator, output) is split into chunks of whole pixels, and a tick
 // packs chunks of any number of requests into one wave of at most kWavePaths (pixel, sample)
 // paths. A tick is a fixed kernel sequence on one stream:
-//   k_primary        camera ray, closest hit, primary shading point per pixel (the GBuffer hit,
-//                    barycentrics rounded to half as the GBuffer stores them, gbuffer.slang:40-60)
+//   k_trace_pixels   camera ray and closest hit per pixel
+//   k_primary        primary shading point per pixel (the GBuffer hit, barycentrics rounded to
+//                    half as the GBuffer stores them, gbuffer.slang:40-60)
 //   k_shade_primary  per path: RNG pcg4d16(pixel, frame, sample), emission on primary, scatter
 //   k = 2..L:        k_trace (closest hit of the ray queue) -> k_shade (emission with MIS,
 //                    roulette, NEE, BSDF sample, ray append) -> k_shadow (any hit of NEE rays)
@@ -39,14 +40,6 @@ static_assert(kWavePaths <= kMaxWavePaths, "path ids must fit the packed queue e
 #define GBPT_SHADE_BLOCKS_PER_SM 5
 #endif
 constexpr int kShadeBlocksPerSM = GBPT_SHADE_BLOCKS_PER_SM;
-// the primary-hit kernel's budget (it traces one camera ray per thread, then shades the hit):
-// 64 registers and some spills beat the 164 registers it takes unbounded (3 blocks per SM) on
-// the 640x360 frame (primary + finalize 0.58 against 0.68 ms; 4 / 6 / 10 / 12 blocks: 0.65 /
-// 0.63 / 0.64 / 0.57)
-#ifndef GBPT_PRIMARY_BLOCKS_PER_SM
-#define GBPT_PRIMARY_BLOCKS_PER_SM 8
-#endif
-constexpr int kPrimaryBlocksPerSM = GBPT_PRIMARY_BLOCKS_PER_SM;
 
 constexpr uint32_t kReqEmission = 1u, kReqNee = 2u, kReqDemodulate = 4u;
 
@@ -119,10 +112,69 @@ GBPT_DI uint32_t chunk_by_path(const ChunkGPU* c, uint32_t n, uint32_t p) {
     return lo;
 }
 
+// Hit records: 2 uint4 per ray, one sector (Work::hit).
+GBPT_DI void store_hit(uint4* hit, uint32_t i, const Hit& h) {
+    hit[2 * i + 0] =
+        make_uint4(__float_as_uint(h.t), __float_as_uint(h.u), __float_as_uint(h.v), h.prim);
+    hit[2 * i + 1] = make_uint4(h.geom, h.inst, 0u, 0u);
+}
+GBPT_DI Hit load_hit(const uint4* hit, uint32_t i) {
+    const uint4 a = hit[2 * i + 0], b = hit[2 * i + 1];
+    Hit h;
+    h.t = __uint_as_float(a.x);
+    h.u = __uint_as_float(a.y);
+    h.v = __uint_as_float(a.z);
+    h.prim = a.w;
+    h.geom = b.x;
+    h.inst = b.y;
+    return h;
+}
+
 GBPT_DI uint32_t pixel_id(const ReqGPU& r, uint32_t li) { return r.pixels ? __ldg(&r.pixels[li]) : li; }
 
-// Primary hit + shading point per pixel slot (gbuffer_rt.slang:18-58, render_pt.slang:98-103)
-__global__ void __launch_bounds__(128, kPrimaryBlocksPerSM) k_primary(TickArgs t, int sort) {
+// The camera ray of pixel slot q: its chunk, direction and span (gbuffer_rt.slang:18-40).
+GBPT_DI const ChunkGPU& slot_ray(const TickArgs& t, uint32_t nc, uint32_t q, float3& o, float3& d,
+                                 float& tmin, float& tmax) {
+    const ChunkGPU& c = t.chunks[chunk_by_slot(t.chunks, nc, q)];
+    const ReqGPU& r = t.reqs[c.req];
+    const uint32_t pid = pixel_id(r, c.pix_first + (q - c.slot_base));
+    camera_ray(r.cam, pid % r.width, pid / r.width, r.width, r.height, o, d, tmin, tmax);
+    return c;
+}
+
+// The primary hit of every pixel slot (persistent warps, counter w.counters[4]), into the hit
+// records at the slot's index. Bound by the traversal's issue slots, like k_trace. The shading
+// point is k_primary's: in one kernel, a thread per pixel, every warp waited for its longest ray
+// and the traversal spilled into the shading's registers (primary hits and shading points of the
+// instanced 1280x720 frame 1.80 instead of 0.36 ms, of the 640x360 soup frame 0.54 instead of
+// 0.21 ms; the frames 8.84 instead of 7.47 and 12.42 instead of 12.11 ms).
+template <bool TWO_LEVEL, bool ALPHA>
+__global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_trace_pixels(TickArgs t) {
+    const uint32_t n = t.hdr->n_pix, nc = t.hdr->n_chunks;
+    auto load = [&](uint32_t i, TraceState& s) {
+        float3 o, d;
+        float tmin, tmax;
+        const ChunkGPU& c = slot_ray(t, nc, i, o, d, tmin, tmax);
+        s.nodes = c.nodes;
+        s.tris_base = c.tris;
+        s.tri_stride = c.tri_stride;
+        s.insts = c.insts;
+        s.mask = c.mask;
+        trace_init(s, o, d, tmin, tmax);
+    };
+    auto store = [&](uint32_t i, const Hit& h) { store_hit(t.w.hit, i, h); };
+    auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
+        return ALPHA && alpha_discard(t.scenes[t.chunks[chunk_by_slot(t.chunks, nc, i)].scene], g,
+                                      p, u, v);
+    };
+    trace_persistent<false, false, TWO_LEVEL>(n, t.w.counters + 4, load, store, alpha, nullptr,
+                                              t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
+}
+
+// The shading point of each pixel slot's primary hit (gbuffer_rt.slang:18-58,
+// render_pt.slang:98-103).
+__global__ void __launch_bounds__(128, kShadeBlocksPerSM) k_primary(TickArgs t, int sort) {
     const uint32_t n = t.hdr->n_pix, nc = t.hdr->n_chunks;
     const uint32_t stride = gridDim.x * blockDim.x;
     // with material-sorted shading: the key of each pixel's primary hit for all its paths
@@ -130,16 +182,12 @@ __global__ void __launch_bounds__(128, kPrimaryBlocksPerSM) k_primary(TickArgs t
     if (threadIdx.x < kSortKeys) key_count[threadIdx.x] = 0u;
     __syncthreads();
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += stride) {
-        const ChunkGPU c = t.chunks[chunk_by_slot(t.chunks, nc, q)];
-        const ReqGPU& r = t.reqs[c.req];
-        const DevScene& sc = t.scenes[c.scene];
-        const uint32_t pid = pixel_id(r, c.pix_first + (q - c.slot_base));
-        const uint32_t px = pid % r.width, py = pid / r.width;
         float3 o, d;
         float tmin, tmax;
-        camera_ray(r.cam, px, py, r.width, r.height, o, d, tmin, tmax);
-        const Hit h = trace_ray<false, false>(sc, o, d, tmin, tmax, c.mask, nullptr,
-                                              t.w.counters + 3);
+        const ChunkGPU& c = slot_ray(t, nc, q, o, d, tmin, tmax);
+        const ReqGPU& r = t.reqs[c.req];
+        const DevScene& sc = t.scenes[c.scene];
+        const Hit h = load_hit(t.w.hit, q);
         if (sort) {
             const uint32_t key = h.geom < sc.geom_count ? __ldg(&c.geom_key[h.geom]) : 0u;
             uint8_t* kp = t.w.keys + c.path_base + (q - c.slot_base) * c.spp;
@@ -176,7 +224,6 @@ __global__ void __launch_bounds__(128, kPrimaryBlocksPerSM) k_primary(TickArgs t
         pc[5] = make_float4(d.x, d.y, d.z, demod.z);
         pc[6] = make_float4(sp.tex_color.x, sp.tex_color.y, sp.tex_color.z, 0.f);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
     if (sort) {
         __syncthreads();
         if (threadIdx.x < kSortKeys && key_count[threadIdx.x])
@@ -333,9 +380,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, kRayTmax);
     };
     auto store = [&](uint32_t i, const Hit& h) {
-        t.w.hit[2 * i + 0] =
-            make_uint4(__float_as_uint(h.t), __float_as_uint(h.u), __float_as_uint(h.v), h.prim);
-        t.w.hit[2 * i + 1] = make_uint4(h.geom, h.inst, 0u, 0u);
+        store_hit(t.w.hit, i, h);
         if (sort) {
             uint32_t key = 0u; // misses shade the environment
             if (h.geom != kNoInst) key = __ldg(&chunk_of(i).geom_key[h.geom]);
@@ -834,6 +879,15 @@ void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int qi
     }
 }
 
+void launch_trace_pixels(const TickArgs& ta, const TickPlan& tp, int grid, cudaStream_t st) {
+    switch ((tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
+    case 0: k_trace_pixels<false, false><<<grid, 128, 0, st>>>(ta); break;
+    case 1: k_trace_pixels<false, true><<<grid, 128, 0, st>>>(ta); break;
+    case 2: k_trace_pixels<true, false><<<grid, 128, 0, st>>>(ta); break;
+    default: k_trace_pixels<true, true><<<grid, 128, 0, st>>>(ta); break;
+    }
+}
+
 void launch_shadow(const TickArgs& ta, const TickPlan& tp, const Grids& g, cudaStream_t st) {
     switch ((tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
     case 0: k_shadow<false, false><<<g.shadow, 128, 0, st>>>(ta); break;
@@ -859,9 +913,12 @@ uint64_t enqueue_tick(const TickArgs& ta, const TickPlan& tp, const Grids& g, cu
     cudaMemsetAsync(ctr, 0, 3 * sizeof(uint32_t), st);
     const int pgrid = (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.primary);
     if (tp.sort) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
+    cudaMemsetAsync(ctr + 4, 0, sizeof(uint32_t), st);
     int ev = prof->begin(st, 3);
+    launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.trace), st);
     k_primary<<<pgrid, 128, 0, st>>>(ta, tp.sort ? 1 : 0);
     prof->end(st, ev);
+    nl += 1;
     const uint32_t* pperm = nullptr;
     if (tp.sort) {
         ev = prof->begin(st, 1);
@@ -1197,6 +1254,7 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     c.nodes = s.nodes;
     c.tris = s.tris;
     c.tri_stride = s.tri_stride;
+    c.insts = s.n_inst ? s.inst : nullptr;
     const TickHeader hdr{1u, P, P, 0u};
     cudaMemcpyAsync(d_reqs, &r, sizeof(r), cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(d_scenes, &s, sizeof(s), cudaMemcpyHostToDevice, st);
@@ -1208,6 +1266,13 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     ta.chunks = d_chunks;
     ta.hdr = d_hdr;
     ta.w = w;
+    const TraceSched sched;
+    ta.refill_lanes = (int)sched.refill_lanes;
+    ta.postpone_lanes = (int)sched.postpone_lanes;
+    const Grids g = launch_grids();
+    TickPlan tp{0, 1, P, P, 1, 1, false, false, s.n_inst != 0u, scene.alpha};
+    cudaMemsetAsync(w.counters + 4, 0, sizeof(uint32_t), st);
+    launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((P + 127) / 128, (uint64_t)g.trace), st);
     k_primary<<<(P + 127) / 128, 128, 0, st>>>(ta, 0);
     // the first 6 float4 of every cached point: the gbpt_debug_primary_points layout
     if (cudaMemcpy2DAsync(out_device, 6 * sizeof(float4), w.pix, kPixFloat4 * sizeof(float4),

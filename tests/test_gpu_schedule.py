@@ -26,3 +26,56 @@ def test_sample_sum_group(gpu_ctx, room, spp, demodulate):
     both = gpu_ctx.render_batch([(sid, cam, p), (sid, cam, big)])
     assert np.isfinite(alone).all() and alone[:, :3].max() > 0
     assert np.array_equal(alone.view(np.uint32), both[0].view(np.uint32))
+
+
+def _scenes():
+    from merian_gb300 import scene as S
+    from merian_gb300 import workloads as W
+    import test_alpha as A
+    return {"room": (S.cornell(), ((0.5, 0.5, -1.4), (0.5, 0.5, 0.0), 40.0)),
+            "instanced": (W.instanced_scene(n_meshes=2, n_u=20, n_v=11, n_instances=30,
+                                            n_textures=2, tex_size=16, box=10.0),
+                          ((5.0, 5.0, -4.5), (5.0, 5.0, 5.0), 60.0)),
+            "alpha": (A.alpha_soup(), ((0.5, 0.5, -0.6), (0.5, 0.5, 0.5), 45.0)),
+            "alpha-instanced": (A.instanced(A.alpha_soup()),
+                                ((2.0, 2.0, -3.0), (2.0, 2.0, 2.0), 60.0))}
+
+
+@pytest.mark.parametrize("kind", ["room", "instanced", "alpha", "alpha-instanced"])
+def test_primary_hits_at_ragged_sizes(gpu_ctx, kind):
+    """Primary hits of images around the sizes of a warp and a block equal the FP32 oracle's bit
+    for bit; the G-buffer, also at a buffer aligned to 4 bytes only, holds the same hits. A ray
+    along a mesh edge (the middle row of pixels in the room) hits two triangles at one
+    t: the kernels take the smaller (geometry, primitive), as the host walk of the same tree does;
+    the oracle's own tree can drop one of the two, and then may only name the larger."""
+    import ctypes as C
+    import torch
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    from oracle import binding as O
+    sc, (pos, target, fov) = _scenes()[kind]
+    osc = O.OracleScene(sc)
+    sid = gpu_ctx.upload(sc)
+    try:
+        for w, h in [(1, 1), (31, 1), (33, 1), (127, 1), (129, 1), (67, 19)]:
+            cam = S.look_at(pos, target, (0.0, 1.0, 0.0), fov, 1.0)
+            g = gpu_ctx.trace_primary(sid, cam, w, h)
+            o, _ = osc.trace_primary(cam, w, h, fp64=False, hit_dtype=N.HIT_DTYPE)
+            assert np.array_equal(g["t"].view(np.uint32), o["t"].view(np.uint32)), (w, h)
+            key = [np.stack([x["instance_index"], x["geometry_index"], x["primitive_id"]], 1)
+                   .astype(np.int64) for x in (g, o)]
+            same = (key[0] == key[1]).all(1)
+            for a, b in zip(key[0][~same], key[1][~same]):
+                assert kind == "room" and tuple(a) < tuple(b)
+            for f in ("instance_id", "barycentrics"):
+                assert np.array_equal(g[f][same].view(np.uint32), o[f][same].view(np.uint32)), f
+            buf = torch.zeros(w * h * 16 + 1, dtype=torch.int32, device="cuda")
+            N.check(gpu_ctx.lib.gbpt_gbuffer(gpu_ctx.handle, sid, C.byref(cam), w, h, 0xFF,
+                                             buf.data_ptr() + 4))
+            gpu_ctx.synchronize()
+            t = np.frombuffer(buf[1:].cpu().numpy().tobytes(), N.GBUFFER_DTYPE)
+            assert np.array_equal(t["primitive_id"], g["primitive_id"])
+            assert np.array_equal(t["geometry_index"],
+                                  (g["geometry_index"] & 0xFFFF).astype(np.uint16))
+    finally:
+        gpu_ctx.destroy_scene(sid)
