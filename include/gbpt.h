@@ -171,7 +171,9 @@ typedef struct gbpt_render_params {
     int32_t emission_on_primary; /* "emission on primary" */
     uint32_t instance_mask;      /* bits "0".."7" */
     int32_t demodulate_albedo;   /* "demodulate albedo" */
-    int32_t sort_materials;      /* "shader execution reordering": material-sorted shading */
+    int32_t sort_materials;      /* "shader execution reordering": a hint without effect on the
+                                    result. The engine sorts by material where that is faster;
+                                    gbpt_tuning.sort_materials forces it on or off */
     uint32_t frame;              /* RNG lane 3, merian's scene.frame ("seed") */
     int32_t nee;                 /* next-event estimation with MIS (0 = BSDF-only estimator) */
     int32_t rr_depth;            /* Russian roulette from this path length (0 = off) */
@@ -328,7 +330,7 @@ GBPT_API int gbpt_set_graphs(gbpt_ctx* ctx, int enable);
  * under every tuning, bit for bit: only the time changes. */
 typedef struct gbpt_tuning {
     uint64_t wave_paths;    /* paths per tick: 0 = default (2^23), else in [1024, 2^24] */
-    int32_t sort_materials; /* -1: as each request's params ask; 0 / 1: force off / on */
+    int32_t sort_materials; /* -1: where the engine finds it faster; 0 / 1: force off / on */
     int32_t use_graphs;     /* gbpt_render_batch replays ticks from CUDA graphs */
     int32_t bvh_build;      /* scenes created after it: GBPT_BVH_* */
     int32_t streams;        /* gbpt_render / gbpt_render_device: 2 (and 0, the default) = ticks

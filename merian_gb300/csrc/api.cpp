@@ -566,14 +566,25 @@ GBPT_API int gbpt_scene_create(gbpt_ctx* ctx, const gbpt_scene_desc* d, uint32_t
         free_scene(s);
         return code;
     };
+    // material-sort key per geometry: 0 environment (UseEnvMap), 1 + min(model, 2) otherwise
+    std::vector<uint8_t> geom_key(std::max<uint32_t>(d->geometry_count, 1u), 0u);
+    for (uint32_t g = 0; g < d->geometry_count; ++g) {
+        const gbpt_geometry& geo = d->geometries[g];
+        if (!(geo.flags & GBPT_MESH_USE_ENV_MAP))
+            geom_key[g] = (uint8_t)(1u + std::min(d->materials[geo.material_id].model, 2u));
+    }
+    for (int k = 1; k <= 3; ++k)
+        s.bsdf_kinds += std::find(geom_key.begin(), geom_key.end(), (uint8_t)k) != geom_key.end();
     if ((rc = upload(&s.nodes, bvh.nodes.data(), bvh.nodes.size() * sizeof(CwNode), bytes))) return fail(rc);
 #if GBPT_TRI_AXIS_COPIES
     {
         // three copies of the records, one after the other, coordinates in the order
         // (c + 1, c + 2, c) mod 3 in copy c (the traversal's watertight test reads copy kz)
+        // and the material-sort key of the geometry in the flag word (kTriKeyShift)
         std::vector<TriRecord> rec(3 * bvh.tris.size());
         for (size_t i = 0; i < bvh.tris.size(); ++i) {
-            const TriRecord& r = bvh.tris[i];
+            TriRecord r = bvh.tris[i];
+            if (r.geom < d->geometry_count) r.pad |= (uint32_t)geom_key[r.geom] << 11;
             for (int c = 0; c < 3; ++c) {
                 TriRecord& o = rec[c * bvh.tris.size() + i];
                 o = r;
@@ -632,16 +643,7 @@ GBPT_API int gbpt_scene_create(gbpt_ctx* ctx, const gbpt_scene_desc* d, uint32_t
                  d->geometries[g].material_id, d->geometries[g].flags};
     if ((rc = upload(&s.geoms, gh.data(), gh.size() * sizeof(GeomHost), bytes))) return fail(rc);
     if ((rc = upload(&s.mats, d->materials, d->material_count * sizeof(gbpt_material), bytes))) return fail(rc);
-    // material-sort key per geometry: 0 environment (UseEnvMap), 1 + min(model, 2) otherwise
-    {
-        std::vector<uint8_t> keys(std::max<uint32_t>(d->geometry_count, 1u), 0u);
-        for (uint32_t g = 0; g < d->geometry_count; ++g) {
-            const gbpt_geometry& geo = d->geometries[g];
-            if (!(geo.flags & GBPT_MESH_USE_ENV_MAP))
-                keys[g] = (uint8_t)(1u + std::min(d->materials[geo.material_id].model, 2u));
-        }
-        if ((rc = upload(&s.geom_key, keys.data(), keys.size(), bytes))) return fail(rc);
-    }
+    if ((rc = upload(&s.geom_key, geom_key.data(), geom_key.size(), bytes))) return fail(rc);
     if (two_level) {
         if ((rc = upload(&s.inst, inst_rec.data(), inst_rec.size() * sizeof(float), bytes))) return fail(rc);
         s.n_inst = d->instance_count;
@@ -956,7 +958,7 @@ static int render_impl(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam,
     RenderArgs a;
     a.camera = *cam;
     a.params = *p;
-    if (ctx->tuning.sort_materials >= 0) a.params.sort_materials = ctx->tuning.sort_materials;
+    a.params.sort_materials = sort_mode(ctx->tuning.sort_materials);
     a.pixel_count = n_pix;
     a.pixels_device = nullptr;
     if (p->pixel_count) {
@@ -1187,8 +1189,7 @@ GBPT_API int gbpt_render_batch(gbpt_ctx* ctx, const gbpt_request* reqs, uint32_t
         const uint32_t np = p.pixel_count ? p.pixel_count : p.width * p.height;
         items[i].camera = reqs[i].camera;
         items[i].params = reqs[i].params;
-        if (ctx->tuning.sort_materials >= 0)
-            items[i].params.sort_materials = ctx->tuning.sort_materials;
+        items[i].params.sort_materials = sort_mode(ctx->tuning.sort_materials);
         items[i].pixel_count = np;
         items[i].pixels_device = nullptr;
         if (p.pixel_count) {

@@ -42,7 +42,7 @@ struct gbpt_ctx {
     cudaStream_t stream2 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // schedule of gbpt_render* and gbpt_render_batch: paths per tick (0 = default), material sort
-    // override (-1 = as each request asks), CUDA graphs
+    // override (-1 = where the engine finds it faster), CUDA graphs
     gbpt_tuning tuning{0, -1, 0, GBPT_BVH_SPLIT, 0, 0, 0, 0};
     // gbpt_autotune's results by (log2 triangles, log2 paths, path length, NEE, roulette depth)
     struct TuneResult {
@@ -71,6 +71,10 @@ namespace gbpt {
 
 // The traversal schedule a tuning asks for (0 fields: the defaults).
 TraceSched sched_of(const gbpt_tuning& t);
+// How the engine orders shading under a tuning's sort_materials (-1: as it finds it faster).
+inline int32_t sort_mode(int32_t tuned) {
+    return tuned < 0 ? kSortAuto : tuned ? kSortOn : kSortOff;
+}
 // Null check and cudaSetDevice for the context's device.
 int check_ctx(gbpt_ctx* ctx);
 // Camera / parameter validation shared by every render entry point.

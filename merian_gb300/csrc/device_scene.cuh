@@ -24,6 +24,8 @@ struct GeomGPU {
 constexpr uint32_t kTriTwoSided = 1u << 8;
 constexpr uint32_t kTriFlip = 1u << 9;
 constexpr uint32_t kTriAlpha = 1u << 10; // non-opaque geometry: candidate hits run the alpha test
+constexpr uint32_t kTriKeyShift = 11;    // material-sort key of the geometry, 2 bits
+constexpr uint32_t kTriKey = 3u << kTriKeyShift;
 
 struct DevScene {
     const uint4* __restrict__ nodes;  // 5 per CWBVH node
@@ -135,7 +137,8 @@ struct RayPre {
     // direction is negative along kz. The watertight test's paper swaps kx and ky for that sign
     // to keep the winding; keeping one frame per kz negates U, V, W, det and T instead, which
     // leaves t, u and v unchanged and flips the facing. The traversal keeps more of the ray in
-    // the same register (set_ray, TraceState): 7 - the direction octant in bits 8-10, the ray's
+    // the same register (set_ray, TraceState): 7 - the direction octant in bits 8-10, the closest
+    // hit's material-sort key in bits 11-12 (kTriKey, as in the triangle's flag word), the ray's
     // instance mask in bits 16-23 and the stack depth in bits 24-31.
     uint32_t k;
     float Sx, Sy, Sz;
@@ -325,9 +328,10 @@ GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
     s.inv = f3(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
     const uint32_t oct = (__float_as_uint(d.x) >> 31) | ((__float_as_uint(d.y) >> 31) << 1) |
                          ((__float_as_uint(d.z) >> 31) << 2);
-    const uint32_t depth = s.pre.k & 0xFF000000u; // the stack outlives a change of space
+    // the stack and the hit outlive a change of space
+    const uint32_t kept = s.pre.k & (0xFF000000u | kTriKey);
     s.pre = ray_pre(o, d);
-    s.pre.k |= ((7u - oct) << 8) | ((s.mask & 0xFFu) << 16) | depth;
+    s.pre.k |= ((7u - oct) << 8) | ((s.mask & 0xFFu) << 16) | kept;
     s.tris = kTriCopies > 1 ? s.tris_base + (size_t)s.pre.kz() * s.tri_stride : s.tris_base;
 }
 
@@ -613,6 +617,7 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
                 s.best.prim = prim;
                 s.best.geom = geom;
                 s.best.inst = s.inst;
+                if (!ANY) s.pre.k = (s.pre.k & ~kTriKey) | (tfl & kTriKey);
                 if (ANY) {
                     done_any = true;
                     break;
@@ -643,7 +648,8 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
 
 // Runs the traversal of every ray i < n with persistent warps that pull ray indices from *fetch
 // (zero before the launch; one atomic per warp for all idle lanes). load(i, state) sets ray i's
-// scene (nodes, tris, insts), mask and calls trace_init; store(i, hit) receives its result;
+// scene (nodes, tris, insts), mask and calls trace_init; store(i, hit, key) receives its result
+// and the material-sort key of the closest hit (0 on a miss);
 // alpha(i, geom, prim, u, v) is ray i's alpha test (true: skip the candidate). Must be called by
 // all 32 lanes of every warp.
 template <bool ANY, bool COUNT, bool TWO_LEVEL, class Load, class Store, class Alpha>
@@ -685,7 +691,7 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
         };
         if (trace_loop<ANY, COUNT, TWO_LEVEL>(s, st_ref, ctr, err, pool_empty, ray_alpha,
                                                     refill_lanes, postpone_lanes)) {
-            store(ray, s.best);
+            store(ray, s.best, (s.pre.k & kTriKey) >> kTriKeyShift);
             active = false;
         }
     }

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         trace_init(s, f3(r.origin[0], r.origin[1], r.origin[2]),
                    f3(r.direction[0], r.direction[1], r.direction[2]), r.tmin, r.tmax);
     };
-    auto store = [&](uint32_t i, const Hit& h) { hits[i] = to_hit(sc, h); };
+    auto store = [&](uint32_t i, const Hit& h, uint32_t) { hits[i] = to_hit(sc, h); };
     auto alpha = [&](uint32_t, uint32_t g, uint32_t p, float u, float v) {
         return alpha_discard(sc, g, p, u, v);
     };
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         s.mask = mask;
         trace_init(s, o, d, tmin, tmax);
     };
-    auto store = [&](uint32_t i, const Hit& ht) {
+    auto store = [&](uint32_t i, const Hit& ht, uint32_t) {
         if (!texels) {
             hits[i] = to_hit(sc, ht);
             return;

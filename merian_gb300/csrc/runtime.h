@@ -75,6 +75,7 @@ struct SceneGPU {
     void* tex_info = nullptr; // uint4 per texture: first texel, width, height, sRGB
     void* srgb_lut = nullptr; // 256 floats
     uint32_t n_tex = 0;
+    int bsdf_kinds = 0; // material-sort keys among the geometries, environment apart
     bool alpha = false; // some geometry is alpha-tested (GBPT_MESH_ALPHA_TEST)
     uint32_t depth = 0;
     uint64_t bytes = 0;
@@ -127,6 +128,10 @@ struct Work {
     // CUDA graphs captured over older buffers are then recaptured
     uint64_t generation = 0;
 };
+
+// How a request's shading is ordered (BatchItem::params.sort_materials): as the engine finds it
+// faster, or always / never by the tuning. Results do not depend on it.
+constexpr int32_t kSortOff = 0, kSortOn = 1, kSortAuto = 2;
 
 // One request of a batch: a scene, a camera, the render parameters and a device output of
 // pixel_count float4 (mean rgb, mean squared luminance), indexed like the pixel list.

@@ -226,7 +226,7 @@ void Server::run() {
             r->item.scene = r->scene;
             r->item.camera = r->req.camera;
             r->item.params = r->req.params;
-            if (sort_override >= 0) r->item.params.sort_materials = sort_override;
+            r->item.params.sort_materials = sort_mode(sort_override);
             r->item.pixel_count = r->n_pix;
             if (r->req.out_host) {
                 r->d_out = (float4*)base;

@@ -44,9 +44,13 @@ constexpr int kShadeBlocksPerSM = GBPT_SHADE_BLOCKS_PER_SM;
 constexpr uint32_t kReqEmission = 1u, kReqNee = 2u, kReqDemodulate = 4u;
 
 // "shader execution reordering" (render_pt.cpp:160-161): the closest-hit queue is ordered by
-// material model before shading, so the warps of k_shade run one BSDF model at a time. Keys:
-// 0 environment (miss or UseEnvMap geometry), 1 diffuse, 2 OpenPBR, 3 OpenPBR with transmission.
-// Shading results do not depend on the order (each entry updates only its own path).
+// material model before shading, so the warps of k_shade run one BSDF model at a time, where that
+// is faster (sorted_vertices) or the tuning asks for it. Keys: 0 environment (miss or UseEnvMap
+// geometry), 1 diffuse, 2 OpenPBR, 3 OpenPBR with transmission; a triangle's flag word carries its
+// key, so the traversal has it without a lookup. The order is the whole queue's, not one of
+// tiles: with tiles of 4,096 entries the warps of one SM ran different models' code at once and
+// the 1080p frame's shading took 77 instead of 51 ms (instruction cache). Shading results do not
+// depend on the order (each entry updates only its own path).
 constexpr int kSortKeys = 4;
 
 struct ReqGPU {
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_trace_pixels(TickArg
         s.mask = c.mask;
         trace_init(s, o, d, tmin, tmax);
     };
-    auto store = [&](uint32_t i, const Hit& h) { store_hit(t.w.hit, i, h); };
+    auto store = [&](uint32_t i, const Hit& h, uint32_t) { store_hit(t.w.hit, i, h); };
     auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(t.scenes[t.chunks[chunk_by_slot(t.chunks, nc, i)].scene], g,
                                       p, u, v);
@@ -359,7 +363,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
     k_trace(TickArgs t, int qi, unsigned long long* work_ctr, int sort) {
     const uint32_t n = t.w.counters[qi];
     TraceCounters ctr{0, 0, 0, 0, 0, 0};
-    // with material-sorted shading: each hit's sort key, counted per block in shared memory
+    // with material-sorted shading: the hits' sort keys, counted per block in shared memory
     __shared__ uint32_t key_count[kSortKeys];
     if (threadIdx.x < kSortKeys) key_count[threadIdx.x] = 0u;
     __syncthreads();
@@ -379,12 +383,10 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         s.mask = c.mask;
         trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, kRayTmax);
     };
-    auto store = [&](uint32_t i, const Hit& h) {
+    auto store = [&](uint32_t i, const Hit& h, uint32_t key) {
         store_hit(t.w.hit, i, h);
         if (sort) {
-            uint32_t key = 0u; // misses shade the environment
-            if (h.geom != kNoInst) key = __ldg(&chunk_of(i).geom_key[h.geom]);
-            t.w.keys[i] = (uint8_t)key;
+            t.w.keys[i] = (uint8_t)key; // misses shade the environment: 0
             atomicAdd(&key_count[key], 1u);
         }
     };
@@ -576,7 +578,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_shadow(TickArgs t) {
         s.mask = c.mask;
         trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, a.w);
     };
-    auto store = [&](uint32_t i, const Hit& h) {
+    auto store = [&](uint32_t i, const Hit& h, uint32_t) {
         if (h.geom == 0xFFFFFFFFu) {
             const uint32_t p = t.w.s_path[i] & kPathMask;
             const float4 c = t.w.s_contrib[i];
@@ -830,12 +832,27 @@ int tables_reserve(Work& w, uint64_t need) {
 }
 
 struct TickPlan {
-    uint32_t chunk_first, n_chunks, n_pix, n_paths, max_len, sum_lanes;
+    uint32_t n_chunks, n_pix, n_paths, max_len, sum_lanes;
+    uint32_t sorted; // material-sorted shading of the path vertices 1..sorted
     bool nee;
-    bool sort; // material-sorted shading (some request asked for it and the Work has the buffers)
     bool two_level; // some chunk's scene is instanced: the two-level traversal variants
     bool alpha;     // some chunk's scene has alpha-tested geometry: the alpha-test variants
 };
+
+// The path vertices whose shading is sorted when the engine chooses: sorting pays where several
+// BSDF models meet in a queue long enough that the warps' divergence costs more than the extra
+// launch and the indirection. The queue's length is known on the device only; it halves about
+// from vertex to vertex (misses, roulette), so vertex k is sorted while paths / 2^(k - 1) is at
+// least 2^16. Measured, shading ms of a frame: 1M-triangle soup at 640x360x16 (3.7 M paths) 4.58
+// unsorted, 2.01 / 1.73 / 1.64 / 1.62 / 1.61 with 2^19 / 2^18 / 2^17 / 2^16 / 2^15; sorting
+// every vertex of short queues cost 37,003 pixels x 8 0.26 instead of 0.24 and a 64x64 frame 0.13
+// instead of 0.09.
+uint32_t sorted_vertices(const TickPlan& tp, int kinds) {
+    uint32_t k = 0;
+    if (kinds > 1)
+        while (k < tp.max_len && k < 31 && (tp.n_paths >> k) >= (1u << 16)) ++k;
+    return k;
+}
 
 // Grid-stride kernels get exactly the blocks that are resident at once: every block strides over
 // the same share of the work, so a second partial wave of blocks would only add a tail.
@@ -864,9 +881,9 @@ Grids launch_grids() {
 // The traversal variants of a tick: work counters, two-level scenes, alpha-tested geometry (the
 // variants without a feature leave its code out; they find the same hits on scenes without it).
 void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int qi,
-                  unsigned long long* work_ctr, cudaStream_t st) {
+                  unsigned long long* work_ctr, bool sort, cudaStream_t st) {
     const int gr = work_ctr ? g.trace_c : g.trace;
-    const int so = tp.sort ? 1 : 0;
+    const int so = sort ? 1 : 0;
     switch ((work_ctr ? 4 : 0) | (tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
     case 0: k_trace<false, false, false><<<gr, 128, 0, st>>>(ta, qi, nullptr, so); break;
     case 1: k_trace<false, false, true><<<gr, 128, 0, st>>>(ta, qi, nullptr, so); break;
@@ -912,15 +929,16 @@ uint64_t enqueue_tick(const TickArgs& ta, const TickPlan& tp, const Grids& g, cu
     uint64_t nl = 0;
     cudaMemsetAsync(ctr, 0, 3 * sizeof(uint32_t), st);
     const int pgrid = (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.primary);
-    if (tp.sort) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
+    const bool sort1 = tp.sorted >= 1;
+    if (sort1) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
     cudaMemsetAsync(ctr + 4, 0, sizeof(uint32_t), st);
     int ev = prof->begin(st, 3);
     launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.trace), st);
-    k_primary<<<pgrid, 128, 0, st>>>(ta, tp.sort ? 1 : 0);
+    k_primary<<<pgrid, 128, 0, st>>>(ta, sort1 ? 1 : 0);
     prof->end(st, ev);
     nl += 1;
     const uint32_t* pperm = nullptr;
-    if (tp.sort) {
+    if (sort1) {
         ev = prof->begin(st, 1);
         k_sort_scatter<<<g.grid / 2, 256, 0, st>>>(ta, -1, ta.w.perm);
         prof->end(st, ev);
@@ -944,12 +962,13 @@ uint64_t enqueue_tick(const TickArgs& ta, const TickPlan& tp, const Grids& g, cu
     for (uint32_t k = 2; k <= L; ++k) {
         const int qo = qi ^ 1;
         cudaMemsetAsync(ctr + 4, 0, sizeof(uint32_t), st);
-        if (tp.sort) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
+        const bool sort = k <= tp.sorted;
+        if (sort) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
         ev = prof->begin(st, 0);
-        launch_trace(ta, tp, g, qi, work_ctr, st);
+        launch_trace(ta, tp, g, qi, work_ctr, sort, st);
         prof->end(st, ev);
         const uint32_t* perm = nullptr;
-        if (tp.sort) {
+        if (sort) {
             ev = prof->begin(st, 1);
             k_sort_scatter<<<g.grid / 2, 256, 0, st>>>(ta, qi, ta.w.perm);
             prof->end(st, ev);
@@ -1038,7 +1057,9 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     DevScene* scenes = (DevScene*)(sb + lay.scenes);
     ChunkGPU* chunks = (ChunkGPU*)(sb + lay.chunks);
     e.scene_ptrs.clear();
-    TickPlan tp{0, 0, 0, 0, 1, 1, false, false, false, false};
+    TickPlan tp{0, 0, 0, 1, 1, 0, false, false, false};
+    int sort_kinds = 0; // BSDF models in one of the scenes
+    bool sort_on = false, sort_auto = false;
     uint64_t paths = 0, pix = 0;
     uint32_t max_spp = 1;
     for (uint32_t i = 0; i < n_items && tp.n_chunks < cap; ++i) {
@@ -1078,7 +1099,9 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
         tp.max_len = std::max(tp.max_len, reqs[ri].max_len);
         max_spp = std::max(max_spp, S);
         tp.nee |= (reqs[ri].flags & kReqNee) != 0u;
-        tp.sort |= it.params.sort_materials != 0;
+        sort_on |= it.params.sort_materials == kSortOn;
+        sort_auto |= it.params.sort_materials == kSortAuto;
+        sort_kinds = std::max(sort_kinds, it.scene->bsdf_kinds);
         it.cursor += (uint32_t)fit;
         if (done && it.cursor == it.pixel_count) done->push_back(i);
     }
@@ -1093,7 +1116,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     // work buffers: a whole wave when graphs replay the tick (their pointers must not move)
     bool graph = e.use_graphs && prof->level == 0;
     if ((rc = work_reserve(w, graph ? wave : paths, graph ? wave : pix)) != GBPT_OK) return rc;
-    tp.sort = tp.sort && w.perm != nullptr;
+    if (w.perm) tp.sorted = sort_on ? tp.max_len : sort_auto ? sorted_vertices(tp, sort_kinds) : 0u;
     unsigned char* tb = (unsigned char*)w.tables;
     if (cudaMemcpyAsync(tb, sb, lay.chunks + tp.n_chunks * sizeof(ChunkGPU), cudaMemcpyHostToDevice,
                         st) != cudaSuccess)
@@ -1125,9 +1148,8 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
             e.release();
             e.graph_generation = w.generation;
         }
-        const uint32_t shape =
-            tp.max_len * 16u + (tp.nee ? 1u : 0u) + (tp.sort ? 2u : 0u) + (tp.two_level ? 4u : 0u) +
-            (tp.alpha ? 8u : 0u);
+        const uint32_t shape = (tp.max_len << 16) + (tp.sorted << 8) + (tp.nee ? 1u : 0u) +
+                               (tp.two_level ? 2u : 0u) + (tp.alpha ? 4u : 0u);
         const TickEngine::Graph* found = nullptr;
         for (const auto& g : e.graphs)
             if (g.shape == shape) found = &g;
@@ -1270,7 +1292,7 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     ta.refill_lanes = (int)sched.refill_lanes;
     ta.postpone_lanes = (int)sched.postpone_lanes;
     const Grids g = launch_grids();
-    TickPlan tp{0, 1, P, P, 1, 1, false, false, s.n_inst != 0u, scene.alpha};
+    TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha};
     cudaMemsetAsync(w.counters + 4, 0, sizeof(uint32_t), st);
     launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((P + 127) / 128, (uint64_t)g.trace), st);
     k_primary<<<(P + 127) / 128, 128, 0, st>>>(ta, 0);

@@ -79,3 +79,23 @@ def test_primary_hits_at_ragged_sizes(gpu_ctx, kind):
                                   (g["geometry_index"] & 0xFFFF).astype(np.uint16))
     finally:
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("paths", [65536 - 256, 65536, 131072 - 256, 131072, 131072 + 256])
+def test_sorted_vertices(gpu_ctx, paths):
+    """The vertices whose shading is sorted depend on the tick's paths (a power of two and its
+    neighbours): the bits of shading that is never and always sorted."""
+    from merian_gb300 import scene as S
+    sc = S.soup(n_triangles=20_000, n_geometries=64, env_size=(64, 32))
+    sid = gpu_ctx.upload(sc)
+    cam = S.look_at((0.5, 0.5, -0.6), (0.5, 0.5, 0.5), (0.0, 1.0, 0.0), 45.0, 1.0)
+    try:
+        p, _ = S.render_params(256, paths // 256, 1, 6, nee=True, rr_depth=3, frame=3)
+        ref = gpu_ctx.render(sid, cam, p)
+        for sort in (0, 1):
+            gpu_ctx.set_tuning(sort_materials=sort)
+            out = gpu_ctx.render(sid, cam, p)
+            assert np.array_equal(ref.view(np.uint32), out.view(np.uint32)), sort
+    finally:
+        gpu_ctx.set_tuning()
+        gpu_ctx.destroy_scene(sid)
