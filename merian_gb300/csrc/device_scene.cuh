@@ -26,6 +26,11 @@ constexpr uint32_t kTriFlip = 1u << 9;
 constexpr uint32_t kTriAlpha = 1u << 10; // non-opaque geometry: candidate hits run the alpha test
 constexpr uint32_t kTriKeyShift = 11;    // material-sort key of the geometry, 2 bits
 constexpr uint32_t kTriKey = 3u << kTriKeyShift;
+constexpr uint32_t kRayAny = 1u << 7;
+
+// What a traversal looks for: every ray's closest hit, every ray's first hit, or per ray the one
+// its axis word says (kRayAny).
+enum TraceMode { kTraceClosest, kTraceAny, kTraceMixed };
 
 struct DevScene {
     const uint4* __restrict__ nodes;  // 5 per CWBVH node
@@ -139,7 +144,8 @@ struct RayPre {
     // leaves t, u and v unchanged and flips the facing. The traversal keeps more of the ray in
     // the same register (set_ray, TraceState): 7 - the direction octant in bits 8-10, the closest
     // hit's material-sort key in bits 11-12 (kTriKey, as in the triangle's flag word), the ray's
-    // instance mask in bits 16-23 and the stack depth in bits 24-31.
+    // instance mask in bits 16-23 and the stack depth in bits 24-31; bit 7 marks a first-hit ray
+    // among closest-hit ones (kRayAny).
     uint32_t k;
     float Sx, Sy, Sz;
     float ox, oy, oz; // origin permuted to (kx, ky, kz)
@@ -329,14 +335,15 @@ GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
     const uint32_t oct = (__float_as_uint(d.x) >> 31) | ((__float_as_uint(d.y) >> 31) << 1) |
                          ((__float_as_uint(d.z) >> 31) << 2);
     // the stack and the hit outlive a change of space
-    const uint32_t kept = s.pre.k & (0xFF000000u | kTriKey);
+    const uint32_t kept = s.pre.k & (0xFF000000u | kTriKey | kRayAny);
     s.pre = ray_pre(o, d);
     s.pre.k |= ((7u - oct) << 8) | ((s.mask & 0xFFu) << 16) | kept;
     s.tris = kTriCopies > 1 ? s.tris_base + (size_t)s.pre.kz() * s.tri_stride : s.tris_base;
 }
 
-GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tmax) {
-    s.pre.k = 0u;
+GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tmax,
+                        uint32_t any = 0u) {
+    s.pre.k = any; // kRayAny or 0
     set_ray(s, o, d);
     s.wo = o;
     s.wd = d;
@@ -511,11 +518,11 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
 }
 
 // Runs the traversal of the ray in s until it is finished (returns true; result in s.best, geom
-// = kNoInst on a miss; with ANY the first hit found) or until the warp should refill its idle
+// = kNoInst on a miss; of a first-hit ray the first hit found) or until the warp should refill its idle
 // lanes (returns false; s keeps the state). `st(i)` is stack entry i. A stack overflow raises *err
 // and finishes the ray with what it found.
 // `alpha(geom, prim, u, v)` decides the candidate hits of non-opaque triangles (true: skip).
-template <bool ANY, bool COUNT, bool TWO_LEVEL, class StackRef, class Alpha>
+template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class StackRef, class Alpha>
 GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32_t* err,
                         bool pool_empty, const Alpha& alpha, int refill_lanes,
                         int postpone_lanes) {
@@ -543,7 +550,7 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
             // the paired planes hold more registers: first-hit traversal, which keeps fewer,
             // measured faster with the scalar ones
             const uint32_t hm =
-                intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && !ANY>(s, ni, cb, tb, im, ctr);
+                intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(s, ni, cb, tb, im, ctr);
             s.ngroup = make_uint2(cb, (hm & 0xFF000000u) | im);
             s.tgroup = make_uint2(tb, hm & 0x00FFFFFFu);
         } else {
@@ -555,7 +562,8 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
         bool done_any = false;
         // only groups followed by node work are postponed (a group popped back is tested), and
         // never those of a first-hit query, which any of its triangles may end
-        const bool may_postpone = !ANY && s.ngroup.y > 0x00FFFFFFu;
+        const bool any = MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u);
+        const bool may_postpone = !any && s.ngroup.y > 0x00FFFFFFu;
         while (s.tgroup.y != 0u) {
             if (may_postpone && s.sp() < kStackSize && __popc(__activemask()) < postpone_lanes) {
                 st(s.sp()) = s.tgroup;
@@ -617,8 +625,8 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
                 s.best.prim = prim;
                 s.best.geom = geom;
                 s.best.inst = s.inst;
-                if (!ANY) s.pre.k = (s.pre.k & ~kTriKey) | (tfl & kTriKey);
-                if (ANY) {
+                if (MODE != kTraceAny) s.pre.k = (s.pre.k & ~kTriKey) | (tfl & kTriKey);
+                if (any) {
                     done_any = true;
                     break;
                 }
@@ -652,7 +660,7 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
 // and the material-sort key of the closest hit (0 on a miss);
 // alpha(i, geom, prim, u, v) is ray i's alpha test (true: skip the candidate). Must be called by
 // all 32 lanes of every warp.
-template <bool ANY, bool COUNT, bool TWO_LEVEL, class Load, class Store, class Alpha>
+template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class Load, class Store, class Alpha>
 __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Load load,
                                                  Store store, Alpha alpha, TraceCounters* ctr,
                                                  uint32_t* err, int refill_lanes,
@@ -689,7 +697,7 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
         const auto ray_alpha = [&](uint32_t g, uint32_t p, float u, float v) {
             return alpha(ray, g, p, u, v);
         };
-        if (trace_loop<ANY, COUNT, TWO_LEVEL>(s, st_ref, ctr, err, pool_empty, ray_alpha,
+        if (trace_loop<MODE, COUNT, TWO_LEVEL>(s, st_ref, ctr, err, pool_empty, ray_alpha,
                                                     refill_lanes, postpone_lanes)) {
             store(ray, s.best, (s.pre.k & kTriKey) >> kTriKeyShift);
             active = false;

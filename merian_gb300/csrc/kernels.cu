@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
     auto alpha = [&](uint32_t, uint32_t g, uint32_t p, float u, float v) {
         return alpha_discard(sc, g, p, u, v);
     };
-    trace_persistent<ANY, true, true>(n, fetch, load, store, alpha, &ctr, err, refill_lanes,
+    trace_persistent<ANY ? kTraceAny : kTraceClosest, true, true>(n, fetch, load, store, alpha, &ctr, err, refill_lanes,
                                       postpone_lanes);
     if (work_ctr) {
         atomicAdd(work_ctr + 0, (unsigned long long)ctr.nodes);
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
     auto alpha = [&](uint32_t, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
-    trace_persistent<false, false, TWO_LEVEL>(w * h, fetch, load, store, alpha, nullptr, err,
+    trace_persistent<kTraceClosest, false, TWO_LEVEL>(w * h, fetch, load, store, alpha, nullptr, err,
                                               refill_lanes, postpone_lanes);
 }
 
@@ -257,13 +257,17 @@ int trace_primary(const SceneGPU& scene, const gbpt_camera& cam, uint32_t w, uin
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 namespace {
-constexpr uint64_t kStaticCounterBytes = 256; // 16 counters + 8 stats words, padded
+// counters and 8 stats words, padded
+constexpr uint64_t kStaticCounterBytes = 1280;
+constexpr uint64_t kStaticStatsAt = 1152;
+static_assert(kCounterWords * 4 <= kStaticStatsAt && kStaticStatsAt + 64 <= kStaticCounterBytes,
+              "static counters");
 constexpr uint64_t kStaticPixelBytes = (uint64_t)kStaticMaxPixelList * 4;
 // per path: throughput and radiance (32), two ray queues (2 x 32), hits (32), shadow queue (52);
 // plus a 112-byte primary point per pixel, budgeted as one pixel per path
 constexpr uint64_t kStaticBytesPerPath = 32 + 2 * 32 + 32 + (32 + 16 + 4) + 16 * kPixFloat4;
 // alignment padding of the carved arrays, and the tick tables of a one-request render
-constexpr uint64_t kStaticSlackBytes = 16 * 256 + 1024;
+constexpr uint64_t kStaticSlackBytes = 16 * 256;
 
 // The array's device address on the current device. Host code cannot use the symbol itself (it
 // names a host-side stand-in), so every call asks the runtime: the lookup allocates nothing, and
@@ -311,7 +315,7 @@ int render_frame_static(const SceneGPU& scene, const RenderArgs& args, const uin
     w.pixel_cap = N;
     unsigned char* p = base;
     w.counters = (uint32_t*)p;
-    w.stats = (unsigned long long*)(p + 64);
+    w.stats = (unsigned long long*)(p + kStaticStatsAt);
     p += kStaticCounterBytes;
     uint32_t* pix_ids = (uint32_t*)p;
     p += kStaticPixelBytes;

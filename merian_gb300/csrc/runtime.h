@@ -81,6 +81,13 @@ struct SceneGPU {
     uint64_t bytes = 0;
 };
 
+// The counters' layout (Work::counters); path lengths go up to 64.
+constexpr uint32_t kMaxVertices = 65;
+constexpr uint32_t kVertexWord = 16;
+constexpr uint32_t kCounterWords = kVertexWord + 4 * kMaxVertices; // of a fixed Work
+constexpr uint32_t kSortWord = kCounterWords;
+constexpr uint32_t kAllCounterWords = kSortWord + 8 * kMaxVertices;
+
 // Work buffers of the wavefront, grown on demand and kept for the context's lifetime.
 // cudaMalloc behind the host-side fault injection of gbpt_debug_fail_allocations (api.cpp). On
 // failure *p is null.
@@ -116,8 +123,11 @@ struct Work {
     uint64_t pix_id_cap = 0;
     float4* out = nullptr;      // device output staging for host-output renders
     uint64_t out_cap = 0;
-    // counters: [0],[1] queue counts, [2] shadow count, [3] error flags, [4],[5] fetch cursors,
-    // [8..11] material-key counts, [12..15] their scatter cursors
+    // counters: [3] error flags; from kVertexWord on, 4 words for every path vertex k of a tick:
+    // the rays and the shadow rays its shading appended, and the fetch cursors of the traversal
+    // that follows (vertex 0: of the primary rays); from kSortWord on (not in a fixed Work),
+    // 8 words per vertex: material-key counts and their scatter cursors. Cleared together at the
+    // start of a tick, the error flags apart
     uint32_t* counters = nullptr;
     unsigned long long* stats = nullptr; // [0] rays, [1] shadow rays, [2] closest-hit rays
     // request, scene and tick tables of the batch being rendered
@@ -209,7 +219,7 @@ struct TickEngine {
     uint64_t graph_generation = 0; // Work::generation the graphs were captured with
     std::vector<unsigned char> stage;
     std::vector<const SceneGPU*> scene_ptrs;
-    int grids[7] = {0, 0, 0, 0, 0, 0, 0}; // launch grids, computed at the first tick
+    int grids[6] = {0, 0, 0, 0, 0, 0}; // launch grids, computed at the first tick
     void release(); // destroys the graphs
 };
 

@@ -9,8 +9,8 @@
 //   k_primary        primary shading point per pixel (the GBuffer hit, barycentrics rounded to
 //                    half as the GBuffer stores them, gbuffer.slang:40-60)
 //   k_shade_primary  per path: RNG pcg4d16(pixel, frame, sample), emission on primary, scatter
-//   k = 2..L:        k_trace (closest hit of the ray queue) -> k_shade (emission with MIS,
-//                    roulette, NEE, BSDF sample, ray append) -> k_shadow (any hit of NEE rays)
+//   k = 2..L:        k_trace (closest hit of the ray queue, any hit of the NEE rays) -> k_shade
+//                    (emission with MIS, roulette, NEE, BSDF sample, ray append)
 //   k_finalize       per pixel: samples summed in a fixed order, NaN/Inf dropped but counted
 // Queue entries carry (chunk << 24 | path), so rays of different scenes share one launch; a
 // chunk holds its scene's traversal pointers. Each pixel's samples live in one tick and are summed
@@ -116,6 +116,13 @@ GBPT_DI uint32_t chunk_by_path(const ChunkGPU* c, uint32_t n, uint32_t p) {
     return lo;
 }
 
+// The counter words of path vertex k (Work::counters).
+enum { kRaysOut = 0, kShadowsOut = 1, kCursor = 2, kCursor2 = 3 };
+GBPT_DI uint32_t* vertex_words(const TickArgs& t, int k) {
+    return t.w.counters + kVertexWord + 4 * k;
+}
+GBPT_DI uint32_t* sort_words(const TickArgs& t, int k) { return t.w.counters + kSortWord + 8 * k; }
+
 // Hit records: 2 uint4 per ray, one sector (Work::hit).
 GBPT_DI void store_hit(uint4* hit, uint32_t i, const Hit& h) {
     hit[2 * i + 0] =
@@ -146,7 +153,7 @@ GBPT_DI const ChunkGPU& slot_ray(const TickArgs& t, uint32_t nc, uint32_t q, flo
     return c;
 }
 
-// The primary hit of every pixel slot (persistent warps, counter w.counters[4]), into the hit
+// The primary hit of every pixel slot (persistent warps, vertex 0's cursor), into the hit
 // records at the slot's index. Bound by the traversal's issue slots, like k_trace. The shading
 // point is k_primary's: in one kernel, a thread per pixel, every warp waited for its longest ray
 // and the traversal spilled into the shading's registers (primary hits and shading points of the
@@ -171,8 +178,9 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_trace_pixels(TickArg
         return ALPHA && alpha_discard(t.scenes[t.chunks[chunk_by_slot(t.chunks, nc, i)].scene], g,
                                       p, u, v);
     };
-    trace_persistent<false, false, TWO_LEVEL>(n, t.w.counters + 4, load, store, alpha, nullptr,
-                                              t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
+    trace_persistent<kTraceClosest, false, TWO_LEVEL>(
+        n, vertex_words(t, 0) + kCursor, load, store, alpha, nullptr, t.w.counters + 3,
+        t.refill_lanes, t.postpone_lanes);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
 }
 
@@ -231,7 +239,7 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM) k_primary(TickArgs t, 
     if (sort) {
         __syncthreads();
         if (threadIdx.x < kSortKeys && key_count[threadIdx.x])
-            atomicAdd(t.w.counters + 8 + threadIdx.x, key_count[threadIdx.x]);
+            atomicAdd(sort_words(t, 1) + threadIdx.x, key_count[threadIdx.x]);
     }
 }
 
@@ -340,13 +348,13 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
             rng_state = rng.state;
         }
         const uint32_t tag = (ci << kPathBits) | p;
-        const uint32_t q = warp_append(t.w.counters + 0, want);
+        const uint32_t q = warp_append(vertex_words(t, 1) + kRaysOut, want);
         if (want) {
             t.w.q_od[0][2 * q + 0] = make_float4(no.x, no.y, no.z, __uint_as_float(rng_state));
             t.w.q_od[0][2 * q + 1] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(tag));
         }
         {
-            const uint32_t sq = warp_append(t.w.counters + 2, want_shadow);
+            const uint32_t sq = warp_append(vertex_words(t, 1) + kShadowsOut, want_shadow);
             if (want_shadow) {
                 t.w.s_od[2 * sq + 0] = s_o;
                 t.w.s_od[2 * sq + 1] = s_d;
@@ -357,49 +365,76 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
     }
 }
 
-// Closest hit for every entry of ray queue `qi` (persistent warps, counter w.counters[4]).
+// The rays that the shading of vertex k appended (persistent warps): the closest hit of every
+// entry of ray queue `qi`, then the occlusion of the shadow queue, whose unoccluded contributions
+// are added to their path (one shadow ray per path and vertex, so no two lanes write the same
+// path; the closest hits touch no path). `parts`: 1 the closest hits, 2 the shadow rays, 3 both in
+// one launch, the longer traversals first.
+// Bound by issue slots (65 % active, 15 of 32 lanes) while the pool lasts, then by the latency of
+// the last rays: one launch has one such tail where a launch for each kind had two (a 64x64 frame
+// 0.28 instead of 0.41 ms, the instanced 1280x720 frame of path length 16 5.6 instead of 7.6, the
+// 640x360 soup frame 8.6 instead of 9.4; the clears of the counters, now one per tick instead of
+// four per vertex, included).
 template <bool COUNT, bool TWO_LEVEL, bool ALPHA>
 __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
-    k_trace(TickArgs t, int qi, unsigned long long* work_ctr, int sort) {
-    const uint32_t n = t.w.counters[qi];
+    k_trace(TickArgs t, int k, int qi, int parts, unsigned long long* work_ctr, int sort) {
+    uint32_t* words = vertex_words(t, k);
+    const uint32_t n_rays = (parts & 1) ? words[kRaysOut] : 0u;
+    const uint32_t n_shadows = (parts & 2) ? words[kShadowsOut] : 0u;
     TraceCounters ctr{0, 0, 0, 0, 0, 0};
     // with material-sorted shading: the hits' sort keys, counted per block in shared memory
     __shared__ uint32_t key_count[kSortKeys];
     if (threadIdx.x < kSortKeys) key_count[threadIdx.x] = 0u;
     __syncthreads();
     const float4* q = t.w.q_od[qi];
-    // the entry's chunk, from the tag in the direction's w
+    // entry i's chunk, from its tag (the direction's w, or the shadow queue's path)
     auto chunk_of = [&](uint32_t i) -> const ChunkGPU& {
-        return t.chunks[__float_as_uint(__ldg((const float*)&q[2 * i + 1] + 3)) >> kPathBits];
+        const uint32_t tag =
+            i < n_rays ? __float_as_uint(__ldg((const float*)&q[2 * i + 1] + 3))
+                       : __ldg(&t.w.s_path[i - n_rays]);
+        return t.chunks[tag >> kPathBits];
     };
     auto load = [&](uint32_t i, TraceState& s) {
-        const float4 a = q[2 * i + 0];
-        const float4 b = q[2 * i + 1];
-        const ChunkGPU& c = t.chunks[__float_as_uint(b.w) >> kPathBits];
+        const bool shadow = i >= n_rays;
+        const float4* e = shadow ? t.w.s_od + 2 * (i - n_rays) : q + 2 * i;
+        const float4 a = e[0], b = e[1];
+        const uint32_t tag = shadow ? __ldg(&t.w.s_path[i - n_rays]) : __float_as_uint(b.w);
+        const ChunkGPU& c = t.chunks[tag >> kPathBits];
         s.nodes = c.nodes;
         s.tris_base = c.tris;
         s.tri_stride = c.tri_stride;
         s.insts = c.insts;
         s.mask = c.mask;
-        trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, kRayTmax);
+        trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, shadow ? a.w : kRayTmax,
+                   shadow ? kRayAny : 0u);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t key) {
-        store_hit(t.w.hit, i, h);
-        if (sort) {
-            t.w.keys[i] = (uint8_t)key; // misses shade the environment: 0
-            atomicAdd(&key_count[key], 1u);
+        if (i < n_rays) {
+            store_hit(t.w.hit, i, h);
+            if (sort) {
+                t.w.keys[i] = (uint8_t)key; // misses shade the environment: 0
+                atomicAdd(&key_count[key], 1u);
+            }
+        } else if (h.geom == kNoInst) {
+            const uint32_t p = t.w.s_path[i - n_rays] & kPathMask;
+            const float4 c = t.w.s_contrib[i - n_rays];
+            float4 r = t.w.path[2 * p + 1];
+            r.x += c.x;
+            r.y += c.y;
+            r.z += c.z;
+            t.w.path[2 * p + 1] = r;
         }
     };
     auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(t.scenes[chunk_of(i).scene], g, p, u, v);
     };
-    trace_persistent<false, COUNT, TWO_LEVEL>(n, t.w.counters + 4, load, store, alpha, &ctr,
-                                              t.w.counters + 3, t.refill_lanes,
-                                              t.postpone_lanes);
+    trace_persistent<kTraceMixed, COUNT, TWO_LEVEL>(
+        n_rays + n_shadows, words + (parts == 2 ? kCursor2 : kCursor), load, store, alpha, &ctr,
+        t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
     if (sort) {
         __syncthreads();
         if (threadIdx.x < kSortKeys && key_count[threadIdx.x])
-            atomicAdd(t.w.counters + 8 + threadIdx.x, key_count[threadIdx.x]);
+            atomicAdd(sort_words(t, k + 1) + threadIdx.x, key_count[threadIdx.x]);
     }
     if (COUNT) {
         atomicAdd(work_ctr + 0, (unsigned long long)ctr.nodes);
@@ -414,15 +449,16 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(t.w.stats + 0, (unsigned long long)n);
-        atomicAdd(t.w.stats + 2, (unsigned long long)n);
+        atomicAdd(t.w.stats + 0, (unsigned long long)n_rays + n_shadows);
+        atomicAdd(t.w.stats + 1, (unsigned long long)n_shadows);
+        atomicAdd(t.w.stats + 2, (unsigned long long)n_rays);
     }
 }
 
 // Emission at the k-th path vertex, then scatter (k < L) into ray queue `qo`.
 __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
     k_shade(TickArgs t, int k, int qi, int qo, const uint32_t* __restrict__ perm) {
-    const uint32_t n = t.w.counters[qi];
+    const uint32_t n = vertex_words(t, k - 1)[kRaysOut];
     const uint32_t stride = gridDim.x * blockDim.x;
     const uint32_t n_round = (n + 31u) & ~31u;
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_round; j += stride) {
@@ -478,13 +514,13 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
             t.w.path[2 * p + 1] = make_float4(rad.x, rad.y, rad.z, last_pdf);
             rng_state = rng.state;
         }
-        const uint32_t q = warp_append(t.w.counters + qo, want);
+        const uint32_t q = warp_append(vertex_words(t, k) + kRaysOut, want);
         if (want) {
             t.w.q_od[qo][2 * q + 0] = make_float4(no.x, no.y, no.z, __uint_as_float(rng_state));
             t.w.q_od[qo][2 * q + 1] = make_float4(nd.x, nd.y, nd.z, __uint_as_float(tag));
         }
         {
-            const uint32_t sq = warp_append(t.w.counters + 2, want_shadow);
+            const uint32_t sq = warp_append(vertex_words(t, k) + kShadowsOut, want_shadow);
             if (want_shadow) {
                 t.w.s_od[2 * sq + 0] = s_o;
                 t.w.s_od[2 * sq + 1] = s_d;
@@ -501,17 +537,19 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
 // writes the permutation. The order of the tiles within a key is not deterministic (shading does
 // not depend on it).
 constexpr uint32_t kSortTile = 2048; // 256 threads x 8 entries
-__global__ void __launch_bounds__(256) k_sort_scatter(TickArgs t, int qi, uint32_t* perm) {
-    const uint32_t n = qi < 0 ? t.hdr->n_paths : t.w.counters[qi]; // qi < 0: the tick's paths
+__global__ void __launch_bounds__(256) k_sort_scatter(TickArgs t, int k, uint32_t* perm) {
+    // the entries shaded at vertex k: the tick's paths, or the rays that reached it
+    const uint32_t n = k == 1 ? t.hdr->n_paths : vertex_words(t, k - 1)[kRaysOut];
+    uint32_t* words = sort_words(t, k);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     __shared__ uint32_t warp_count[8][kSortKeys]; // then each warp's offset within the tile
     __shared__ uint32_t tile_base[kSortKeys];
     uint32_t key_base[kSortKeys];
     uint32_t acc = 0;
 #pragma unroll
-    for (int k = 0; k < kSortKeys; ++k) {
-        key_base[k] = acc;
-        acc += t.w.counters[8 + k];
+    for (int j = 0; j < kSortKeys; ++j) {
+        key_base[j] = acc;
+        acc += words[j];
     }
     for (uint32_t tile = blockIdx.x; tile * kSortTile < n; tile += gridDim.x) {
         // this warp's 256 consecutive entries: 8 rounds of 32
@@ -535,14 +573,14 @@ __global__ void __launch_bounds__(256) k_sort_scatter(TickArgs t, int qi, uint32
         }
         __syncthreads();
         if (threadIdx.x < kSortKeys) {
-            const uint32_t k = threadIdx.x;
+            const uint32_t j = threadIdx.x;
             uint32_t run = 0;
             for (int w = 0; w < 8; ++w) {
-                const uint32_t c = warp_count[w][k];
-                warp_count[w][k] = run;
+                const uint32_t c = warp_count[w][j];
+                warp_count[w][j] = run;
                 run += c;
             }
-            tile_base[k] = run ? key_base[k] + atomicAdd(t.w.counters + 12 + k, run) : 0u;
+            tile_base[j] = run ? key_base[j] + atomicAdd(words + kSortKeys + j, run) : 0u;
         }
         __syncthreads();
         uint32_t at[kSortKeys];
@@ -559,45 +597,6 @@ __global__ void __launch_bounds__(256) k_sort_scatter(TickArgs t, int qi, uint32
             }
         }
         __syncthreads(); // warp_count and tile_base are reused by the next tile
-    }
-}
-
-// Occlusion of the NEE queue; unoccluded contributions are added to their path (one shadow ray
-// per path per bounce, so no two lanes write the same path).
-template <bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_shadow(TickArgs t) {
-    const uint32_t n = t.w.counters[2];
-    auto load = [&](uint32_t i, TraceState& s) {
-        const ChunkGPU& c = t.chunks[__ldg(&t.w.s_path[i]) >> kPathBits];
-        const float4 a = t.w.s_od[2 * i + 0];
-        const float4 b = t.w.s_od[2 * i + 1];
-        s.nodes = c.nodes;
-        s.tris_base = c.tris;
-        s.tri_stride = c.tri_stride;
-        s.insts = c.insts;
-        s.mask = c.mask;
-        trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, a.w);
-    };
-    auto store = [&](uint32_t i, const Hit& h, uint32_t) {
-        if (h.geom == 0xFFFFFFFFu) {
-            const uint32_t p = t.w.s_path[i] & kPathMask;
-            const float4 c = t.w.s_contrib[i];
-            float4 r = t.w.path[2 * p + 1];
-            r.x += c.x;
-            r.y += c.y;
-            r.z += c.z;
-            t.w.path[2 * p + 1] = r;
-        }
-    };
-    auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
-        return ALPHA && alpha_discard(t.scenes[t.chunks[__ldg(&t.w.s_path[i]) >> kPathBits].scene],
-                                      g, p, u, v);
-    };
-    trace_persistent<true, false, TWO_LEVEL>(n, t.w.counters + 5, load, store, alpha, nullptr,
-                                             t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(t.w.stats + 0, (unsigned long long)n);
-        atomicAdd(t.w.stats + 1, (unsigned long long)n);
     }
 }
 
@@ -735,13 +734,13 @@ int work_reserve(Work& w, uint64_t paths, uint64_t pixels) {
         uint64_t b = 0;
         release(w.counters);
         release(w.stats);
-        if (alloc(w.counters, 16, b) != cudaSuccess || alloc(w.stats, 8, b) != cudaSuccess) {
+        if (alloc(w.counters, kAllCounterWords, b) != cudaSuccess || alloc(w.stats, 8, b) != cudaSuccess) {
             release(w.counters);
             release(w.stats);
             return GBPT_ERR_NO_MEMORY;
         }
         new_generation(w);
-        cudaMemset(w.counters, 0, 16 * sizeof(uint32_t));
+        cudaMemset(w.counters, 0, kAllCounterWords * sizeof(uint32_t));
         cudaMemset(w.stats, 0, 8 * sizeof(unsigned long long));
         w.bytes += b;
     }
@@ -860,7 +859,6 @@ struct Grids {
     int grid;    // grid-stride kernels without a register budget (finalize, material sort)
     int trace;   // persistent traversal: the blocks resident at once
     int trace_c;
-    int shadow;
     int primary; // k_primary, k_shade_primary, k_shade: their resident blocks
     int shade_p;
     int shade;
@@ -871,7 +869,6 @@ Grids launch_grids() {
     // the two-level and alpha variants have the same launch bounds, hence the same residency
     g.trace = persistent_grid(k_trace<false, false, false>);
     g.trace_c = persistent_grid(k_trace<true, false, false>);
-    g.shadow = persistent_grid(k_shadow<false, false>);
     g.primary = persistent_grid(k_primary);
     g.shade_p = persistent_grid(k_shade_primary);
     g.shade = persistent_grid(k_shade);
@@ -880,19 +877,20 @@ Grids launch_grids() {
 
 // The traversal variants of a tick: work counters, two-level scenes, alpha-tested geometry (the
 // variants without a feature leave its code out; they find the same hits on scenes without it).
-void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int qi,
+void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k, int qi, int parts,
                   unsigned long long* work_ctr, bool sort, cudaStream_t st) {
     const int gr = work_ctr ? g.trace_c : g.trace;
     const int so = sort ? 1 : 0;
+    auto go = [&](auto kernel) { kernel<<<gr, 128, 0, st>>>(ta, k, qi, parts, work_ctr, so); };
     switch ((work_ctr ? 4 : 0) | (tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
-    case 0: k_trace<false, false, false><<<gr, 128, 0, st>>>(ta, qi, nullptr, so); break;
-    case 1: k_trace<false, false, true><<<gr, 128, 0, st>>>(ta, qi, nullptr, so); break;
-    case 2: k_trace<false, true, false><<<gr, 128, 0, st>>>(ta, qi, nullptr, so); break;
-    case 3: k_trace<false, true, true><<<gr, 128, 0, st>>>(ta, qi, nullptr, so); break;
-    case 4: k_trace<true, false, false><<<gr, 128, 0, st>>>(ta, qi, work_ctr, so); break;
-    case 5: k_trace<true, false, true><<<gr, 128, 0, st>>>(ta, qi, work_ctr, so); break;
-    case 6: k_trace<true, true, false><<<gr, 128, 0, st>>>(ta, qi, work_ctr, so); break;
-    default: k_trace<true, true, true><<<gr, 128, 0, st>>>(ta, qi, work_ctr, so); break;
+    case 0: go(k_trace<false, false, false>); break;
+    case 1: go(k_trace<false, false, true>); break;
+    case 2: go(k_trace<false, true, false>); break;
+    case 3: go(k_trace<false, true, true>); break;
+    case 4: go(k_trace<true, false, false>); break;
+    case 5: go(k_trace<true, false, true>); break;
+    case 6: go(k_trace<true, true, false>); break;
+    default: go(k_trace<true, true, true>); break;
     }
 }
 
@@ -905,90 +903,65 @@ void launch_trace_pixels(const TickArgs& ta, const TickPlan& tp, int grid, cudaS
     }
 }
 
-void launch_shadow(const TickArgs& ta, const TickPlan& tp, const Grids& g, cudaStream_t st) {
-    switch ((tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
-    case 0: k_shadow<false, false><<<g.shadow, 128, 0, st>>>(ta); break;
-    case 1: k_shadow<false, true><<<g.shadow, 128, 0, st>>>(ta); break;
-    case 2: k_shadow<true, false><<<g.shadow, 128, 0, st>>>(ta); break;
-    default: k_shadow<true, true><<<g.shadow, 128, 0, st>>>(ta); break;
-    }
-}
-
-// The kernel sequence of one tick; returns the number of kernel launches. Counter words
-// ([0], [1] ray queues, [2] shadow queue, [4], [5] fetch cursors) are cleared on the stream
-// before their producer runs; the error flag ([3]) is left for the caller to read.
+// The kernel sequence of one tick; returns the number of kernel launches. The vertices' counter
+// words are cleared once, before the first kernel; the error flag ([3]) is left for the caller to
+// read. While profiling, closest hits and shadow rays are launched apart, to be timed apart.
 // With fixed_grid every launch gets the full grid whatever the tick's size (a graph replays any
 // tick of the same shape); the kernels stride over the sizes in the tick header.
 uint64_t enqueue_tick(const TickArgs& ta, const TickPlan& tp, const Grids& g, cudaStream_t st,
                       Profile* prof, unsigned long long* work_ctr, bool fixed_grid) {
     uint32_t* ctr = ta.w.counters;
-    const bool nee = tp.nee;
     const uint32_t L = tp.max_len;
     const uint64_t pix = fixed_grid ? ~0ull >> 8 : tp.n_pix;
     const uint64_t paths = fixed_grid ? ~0ull >> 8 : tp.n_paths;
     uint64_t nl = 0;
-    cudaMemsetAsync(ctr, 0, 3 * sizeof(uint32_t), st);
+    cudaMemsetAsync(ctr + kVertexWord, 0, (L + 1) * 4 * sizeof(uint32_t), st);
+    if (tp.sorted)
+        cudaMemsetAsync(ctr + kSortWord, 0, (tp.sorted + 1) * 8 * sizeof(uint32_t), st);
     const int pgrid = (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.primary);
-    const bool sort1 = tp.sorted >= 1;
-    if (sort1) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
-    cudaMemsetAsync(ctr + 4, 0, sizeof(uint32_t), st);
     int ev = prof->begin(st, 3);
     launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.trace), st);
-    k_primary<<<pgrid, 128, 0, st>>>(ta, sort1 ? 1 : 0);
-    prof->end(st, ev);
-    nl += 1;
-    const uint32_t* pperm = nullptr;
-    if (sort1) {
-        ev = prof->begin(st, 1);
-        k_sort_scatter<<<g.grid / 2, 256, 0, st>>>(ta, -1, ta.w.perm);
-        prof->end(st, ev);
-        pperm = ta.w.perm;
-        nl += 1;
-    }
-    const int sgrid = (int)std::min<uint64_t>((paths + 127) / 128, (uint64_t)g.shade_p);
-    ev = prof->begin(st, 1);
-    k_shade_primary<<<sgrid, 128, 0, st>>>(ta, pperm);
+    k_primary<<<pgrid, 128, 0, st>>>(ta, tp.sorted >= 1 ? 1 : 0);
     prof->end(st, ev);
     nl += 2;
-    if (nee) {
-        cudaMemsetAsync(ctr + 5, 0, sizeof(uint32_t), st);
-        ev = prof->begin(st, 2);
-        launch_shadow(ta, tp, g, st);
+    auto sorted = [&](uint32_t k) -> const uint32_t* {
+        if (k > tp.sorted) return nullptr;
+        ev = prof->begin(st, 1);
+        k_sort_scatter<<<g.grid / 2, 256, 0, st>>>(ta, (int)k, ta.w.perm);
         prof->end(st, ev);
-        cudaMemsetAsync(ctr + 2, 0, sizeof(uint32_t), st);
         nl += 1;
-    }
+        return ta.w.perm;
+    };
+    const int sgrid = (int)std::min<uint64_t>((paths + 127) / 128, (uint64_t)g.shade_p);
+    const uint32_t* perm = sorted(1);
+    ev = prof->begin(st, 1);
+    k_shade_primary<<<sgrid, 128, 0, st>>>(ta, perm);
+    prof->end(st, ev);
+    nl += 1;
     int qi = 0;
     for (uint32_t k = 2; k <= L; ++k) {
-        const int qo = qi ^ 1;
-        cudaMemsetAsync(ctr + 4, 0, sizeof(uint32_t), st);
         const bool sort = k <= tp.sorted;
-        if (sort) cudaMemsetAsync(ctr + 8, 0, 8 * sizeof(uint32_t), st); // key counts, cursors
-        ev = prof->begin(st, 0);
-        launch_trace(ta, tp, g, qi, work_ctr, sort, st);
-        prof->end(st, ev);
-        const uint32_t* perm = nullptr;
-        if (sort) {
-            ev = prof->begin(st, 1);
-            k_sort_scatter<<<g.grid / 2, 256, 0, st>>>(ta, qi, ta.w.perm);
+        if (prof->level == 0) {
+            launch_trace(ta, tp, g, (int)k - 1, qi, tp.nee ? 3 : 1, nullptr, sort, st);
+            nl += 1;
+        } else {
+            if (tp.nee) {
+                ev = prof->begin(st, 2);
+                launch_trace(ta, tp, g, (int)k - 1, qi, 2, nullptr, false, st);
+                prof->end(st, ev);
+                nl += 1;
+            }
+            ev = prof->begin(st, 0);
+            launch_trace(ta, tp, g, (int)k - 1, qi, 1, work_ctr, sort, st);
             prof->end(st, ev);
-            perm = ta.w.perm;
             nl += 1;
         }
-        cudaMemsetAsync(ctr + qo, 0, sizeof(uint32_t), st);
+        perm = sorted(k);
         ev = prof->begin(st, 1);
-        k_shade<<<g.shade, 128, 0, st>>>(ta, (int)k, qi, qo, perm);
+        k_shade<<<g.shade, 128, 0, st>>>(ta, (int)k, qi, qi ^ 1, perm);
         prof->end(st, ev);
-        nl += 2;
-        if (nee && k < L) {
-            cudaMemsetAsync(ctr + 5, 0, sizeof(uint32_t), st);
-            ev = prof->begin(st, 2);
-            launch_shadow(ta, tp, g, st);
-            prof->end(st, ev);
-            cudaMemsetAsync(ctr + 2, 0, sizeof(uint32_t), st);
-            nl += 1;
-        }
-        qi = qo;
+        nl += 1;
+        qi ^= 1;
     }
     ev = prof->begin(st, 3);
     k_finalize<<<(int)std::min<uint64_t>((pix * tp.sum_lanes + 127) / 128, (uint64_t)g.grid), 128, 0,
@@ -1140,7 +1113,6 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
         const int cap = (int)e.sched.blocks_per_sm * num_sms();
         grids.trace = std::min(grids.trace, cap);
         grids.trace_c = std::min(grids.trace_c, cap);
-        grids.shadow = std::min(grids.shadow, cap);
     }
     uint64_t nl = 0;
     if (graph) {
@@ -1293,7 +1265,7 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     ta.postpone_lanes = (int)sched.postpone_lanes;
     const Grids g = launch_grids();
     TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha};
-    cudaMemsetAsync(w.counters + 4, 0, sizeof(uint32_t), st);
+    cudaMemsetAsync(w.counters + kVertexWord, 0, 4 * sizeof(uint32_t), st);
     launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((P + 127) / 128, (uint64_t)g.trace), st);
     k_primary<<<(P + 127) / 128, 128, 0, st>>>(ta, 0);
     // the first 6 float4 of every cached point: the gbpt_debug_primary_points layout

@@ -99,3 +99,29 @@ def test_sorted_vertices(gpu_ctx, paths):
     finally:
         gpu_ctx.set_tuning()
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("kind", ["room", "instanced", "alpha", "alpha-instanced"])
+def test_closest_and_shadow_rays_in_one_launch(gpu_ctx, kind):
+    """A vertex's bounce rays and shadow rays share one traversal launch; profiling launches them
+    apart. Same bits and ray counts, around the sizes of a warp and a block."""
+    from merian_gb300 import scene as S
+    sc, (pos, target, fov) = _scenes()[kind]
+    if sc.env is None:
+        sc.env = np.ones((8, 16, 4), np.float32)
+    sid = gpu_ctx.upload(sc)
+    cam = S.look_at(pos, target, (0.0, 1.0, 0.0), fov, 1.0)
+    try:
+        for w, h, spp in [(1, 1, 1), (31, 1, 1), (33, 1, 1), (43, 3, 1), (61, 37, 5)]:
+            p, _ = S.render_params(w, h, spp, 6, nee=True, rr_depth=3, frame=w)
+            a, sa = gpu_ctx.render(sid, cam, p, stats=True)
+            gpu_ctx.set_profiling(1)
+            b, sb = gpu_ctx.render(sid, cam, p, stats=True)
+            gpu_ctx.set_profiling(0)
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (w, h)
+            assert (sa.rays, sa.shadow_rays, sa.trace_rays) == (sb.rays, sb.shadow_rays,
+                                                                sb.trace_rays)
+            assert sa.kernel_launches < sb.kernel_launches
+    finally:
+        gpu_ctx.set_profiling(0)
+        gpu_ctx.destroy_scene(sid)
