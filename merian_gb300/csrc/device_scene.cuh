@@ -311,7 +311,6 @@ struct TraceState {
     const float4* tris_base; // copy 0 of the records and the float4 from one copy to the next
     uint32_t tri_stride;
     const float4* insts; // instance records; nullptr for single-level scenes
-    uint32_t mask;       // instance mask of the ray
     float3 o, d, inv;    // the ray in the current space (object space inside an instance)
     float tmin;
     RayPre pre;
@@ -321,6 +320,11 @@ struct TraceState {
     float3 wo, wd; // the world ray
     uint32_t inst; // instance being traversed, kNoInst at the top level
     int inst_sp;   // stack depth at which it was entered
+    // bits 0-7: the stack's first entry of this lane (those below were given to other lanes);
+    // bits 8-12: the lane that keeps the ray's result; bits 16 up: steps of the current run
+    uint32_t aux;
+    GBPT_DI int floor() const { return (int)(aux & 0xFFu); }
+    GBPT_DI uint32_t owner() const { return (aux >> 8) & 31u; }
     // the traversal stack's depth, kept in bits 24..31 of the ray's axis word
     GBPT_DI int sp() const { return (int)(pre.k >> 24); }
     GBPT_DI void push_sp() { pre.k += 1u << 24; }
@@ -334,16 +338,16 @@ GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
     s.inv = f3(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
     const uint32_t oct = (__float_as_uint(d.x) >> 31) | ((__float_as_uint(d.y) >> 31) << 1) |
                          ((__float_as_uint(d.z) >> 31) << 2);
-    // the stack and the hit outlive a change of space
-    const uint32_t kept = s.pre.k & (0xFF000000u | kTriKey | kRayAny);
+    // the stack, the mask and the hit outlive a change of space
+    const uint32_t kept = s.pre.k & (0xFFFF0000u | kTriKey | kRayAny);
     s.pre = ray_pre(o, d);
-    s.pre.k |= ((7u - oct) << 8) | ((s.mask & 0xFFu) << 16) | kept;
+    s.pre.k |= ((7u - oct) << 8) | kept;
     s.tris = kTriCopies > 1 ? s.tris_base + (size_t)s.pre.kz() * s.tri_stride : s.tris_base;
 }
 
-GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tmax,
+GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tmax, uint32_t mask,
                         uint32_t any = 0u) {
-    s.pre.k = any; // kRayAny or 0
+    s.pre.k = ((mask & 0xFFu) << 16) | any; // any: kRayAny or 0
     set_ray(s, o, d);
     s.wo = o;
     s.wd = d;
@@ -524,7 +528,7 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
 // `alpha(geom, prim, u, v)` decides the candidate hits of non-opaque triangles (true: skip).
 template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class StackRef, class Alpha>
 GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32_t* err,
-                        bool pool_empty, const Alpha& alpha, int refill_lanes,
+                        const Alpha& alpha, int min_lanes, uint32_t step_mask,
                         int postpone_lanes) {
     while (true) {
         if (s.ngroup.y > 0x00FFFFFFu) {
@@ -635,7 +639,7 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
         bool done = done_any;
         if (!done && s.ngroup.y <= 0x00FFFFFFu) {
             if (TWO_LEVEL && s.inst != kNoInst && s.sp() == s.inst_sp) exit_instance(s);
-            if (s.sp() == 0) {
+            if (s.sp() == s.floor()) {
                 done = true;
             } else {
                 s.pop_sp();
@@ -643,64 +647,244 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
             }
         }
         if (done) break;
-        if (!pool_empty && __popc(__activemask()) < refill_lanes) return false;
+        s.aux += 1u << 16;
+        if ((s.aux & step_mask) == 0u && __popc(__activemask()) < min_lanes) return false;
     }
-#if GBPT_DEFER_UV
-    if (s.best.geom != kNoInst) {
-        s.best.u = __fdiv_rn(s.best.u, s.det);
-        s.best.v = __fdiv_rn(s.best.v, s.det);
-    }
-#endif
     return true;
+}
+
+// Position of the r-th set bit of m (r < popc(m)).
+GBPT_DI uint32_t nth_bit(uint32_t m, uint32_t r) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (uint32_t w = 16; w > 0; w >>= 1) {
+        const uint32_t c = __popc((m >> pos) & ((1u << w) - 1u));
+        if (r >= c) {
+            r -= c;
+            pos += w;
+        }
+    }
+    return pos;
+}
+
+template <class T> GBPT_DI T* shfl_ptr(T* p, uint32_t src) {
+    return (T*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)p, src);
+}
+
+// Whether hit a comes before b: nearer, or at the same distance the smaller (geometry, primitive,
+// instance).
+GBPT_DI bool hit_before(float t, uint32_t geom, uint32_t prim, uint32_t inst, const Hit& b) {
+    return t < b.t || (t == b.t && (geom < b.geom ||
+                                    (geom == b.geom &&
+                                     (prim < b.prim || (prim == b.prim && inst < b.inst)))));
+}
+
+// Once the pool is empty, the rays a warp has left are shared out: idle lanes take the oldest stack
+// entries of busy ones and traverse them for the same ray (helpers). The lane that loaded the ray
+// (its owner) keeps the result: helpers report hits to it and take over its distance, and it
+// stores the result when no lane works on the ray any more. The closest hit and the tie rule do
+// not depend on which lane finds it. Called by all 32 lanes; `active`: the lane traverses a part
+// of a ray; `owns`: it keeps an unfinished ray.
+// One long ray (a hundred dependent node steps of about a microsecond each) used to keep its warp,
+// and with it the launch, while 31 lanes idled: without / with sharing, the instanced 1280x720
+// frame of path length 16 takes 5.56 / 4.41 ms, 37,003 pixels x 8 of the 200k-triangle soup 2.17 /
+// 1.79, a 64x64 frame of the room 0.30 / 0.25; where queues are long it is neutral (1080p soup
+// frame 261.5 / 260.6).
+// Steps between two shares: 1 / 2 / 4 / 8 measure 4.31 / 4.41 / 4.53 / 4.74 ms on the instanced
+// frame, 1.81 / 1.79 / 1.79 / 1.86 on the pixel list, 260.6 / 260.8 / 261.5 (2 / 4 / 8) on the 1080p
+// soup.
+constexpr uint32_t kShareSteps = 2; // a power of two
+template <TraceMode MODE, bool TWO_LEVEL, class StackRef, class Store>
+GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& active, bool& owns,
+                        const Store& store) {
+    const uint32_t lane = threadIdx.x & 31u;
+    // helpers' hits, one at a time, to their rays' owners
+    const bool helper = s.owner() != lane;
+    uint32_t m = __ballot_sync(0xFFFFFFFFu, helper && s.best.geom != kNoInst);
+    while (m != 0u) {
+        const uint32_t h = __ffs(m) - 1u;
+        m &= m - 1u;
+        const uint32_t o = __shfl_sync(0xFFFFFFFFu, s.owner(), h);
+        const float t = __shfl_sync(0xFFFFFFFFu, s.best.t, h);
+        const float u = __shfl_sync(0xFFFFFFFFu, s.best.u, h);
+        const float v = __shfl_sync(0xFFFFFFFFu, s.best.v, h);
+        const float det = __shfl_sync(0xFFFFFFFFu, s.det, h);
+        const uint32_t prim = __shfl_sync(0xFFFFFFFFu, s.best.prim, h);
+        const uint32_t geom = __shfl_sync(0xFFFFFFFFu, s.best.geom, h);
+        const uint32_t inst = TWO_LEVEL ? __shfl_sync(0xFFFFFFFFu, s.best.inst, h) : kNoInst;
+        const uint32_t k = __shfl_sync(0xFFFFFFFFu, s.pre.k, h);
+        if (lane == o && hit_before(t, geom, prim, inst, s.best)) {
+            s.best.t = t;
+            s.best.u = u;
+            s.best.v = v;
+            s.det = det;
+            s.best.prim = prim;
+            s.best.geom = geom;
+            s.best.inst = inst;
+            s.pre.k = (s.pre.k & ~kTriKey) | (k & kTriKey);
+        }
+        if (lane == h) s.best.prim = s.best.geom = s.best.inst = kNoInst;
+    }
+    // the owner's distance; a first-hit ray ends with its first hit
+    const float t_own = __shfl_sync(0xFFFFFFFFu, s.best.t, s.owner());
+    const uint32_t g_own = __shfl_sync(0xFFFFFFFFu, s.best.geom, s.owner());
+    if (helper) s.best.t = fminf(s.best.t, t_own);
+    const bool any =
+        MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u);
+    if (any && g_own != kNoInst) active = false;
+    // rays without a busy lane
+    const uint32_t busy = __reduce_or_sync(0xFFFFFFFFu, active ? 1u << s.owner() : 0u);
+    if (owns && ((busy >> lane) & 1u) == 0u) {
+        store(ray, s);
+        owns = false;
+    }
+    // idle lanes take stack entries
+    const bool donor = active && s.sp() > s.floor();
+    const bool idle = !active && !owns;
+    const uint32_t m_donor = __ballot_sync(0xFFFFFFFFu, donor);
+    const uint32_t m_idle = __ballot_sync(0xFFFFFFFFu, idle);
+    const uint32_t pairs = min(__popc(m_donor), __popc(m_idle));
+    if (pairs == 0u) return;
+    const uint32_t below = (1u << lane) - 1u;
+    uint2 e = make_uint2(0u, 0u);
+    bool top = false; // the entry belongs to the top level while the donor is in an instance
+    if (donor && __popc(m_donor & below) < pairs) {
+        e = st(s.floor());
+        top = TWO_LEVEL && s.inst != kNoInst && s.floor() < s.inst_sp;
+        s.aux += 1u;
+    }
+    const uint32_t r = __popc(m_idle & below);
+    const bool take = idle && r < pairs;
+    const uint32_t src = take ? nth_bit(m_donor, r) : lane;
+    auto f = [&](float x) { return __shfl_sync(0xFFFFFFFFu, x, src); };
+    auto w = [&](uint32_t x) { return __shfl_sync(0xFFFFFFFFu, x, src); };
+    s.nodes = shfl_ptr(s.nodes, src);
+    s.tris = shfl_ptr(s.tris, src);
+    s.o = f3(f(s.o.x), f(s.o.y), f(s.o.z));
+    s.inv = f3(f(s.inv.x), f(s.inv.y), f(s.inv.z));
+    s.tmin = f(s.tmin);
+    s.pre.Sx = f(s.pre.Sx);
+    s.pre.Sy = f(s.pre.Sy);
+    s.pre.Sz = f(s.pre.Sz);
+    s.pre.ox = f(s.pre.ox);
+    s.pre.oy = f(s.pre.oy);
+    s.pre.oz = f(s.pre.oz);
+    s.best.t = f(s.best.t);
+    ray = w(ray);
+    const uint32_t k = w(s.pre.k), aux = w(s.aux);
+    e.x = w(e.x);
+    e.y = w(e.y);
+    bool restart = false;
+    if (TWO_LEVEL) {
+        s.tris_base = shfl_ptr(s.tris_base, src);
+        s.tri_stride = w(s.tri_stride);
+        s.insts = shfl_ptr(s.insts, src);
+        s.wo = f3(f(s.wo.x), f(s.wo.y), f(s.wo.z));
+        s.wd = f3(f(s.wd.x), f(s.wd.y), f(s.wd.z));
+        s.inst = w(s.inst);
+        restart = w(top ? 1u : 0u) != 0u;
+    }
+    if (take) {
+        active = true;
+        s.pre.k = k & ~(0xFF000000u | kTriKey); // an empty stack, no hit
+        s.aux = aux & 0x1F00u;
+        s.ngroup = e;
+        s.tgroup = make_uint2(0u, 0u);
+        s.best.prim = s.best.geom = s.best.inst = kNoInst;
+        s.inst_sp = TWO_LEVEL && s.inst != kNoInst ? 0 : -1;
+        if (TWO_LEVEL && restart) exit_instance(s);
+    }
 }
 
 // Runs the traversal of every ray i < n with persistent warps that pull ray indices from *fetch
 // (zero before the launch; one atomic per warp for all idle lanes). load(i, state) sets ray i's
-// scene (nodes, tris, insts), mask and calls trace_init; store(i, hit, key) receives its result
+// scene (nodes, tris, insts) and calls trace_init; store(i, hit, key) receives its result
 // and the material-sort key of the closest hit (0 on a miss);
 // alpha(i, geom, prim, u, v) is ray i's alpha test (true: skip the candidate). Must be called by
-// all 32 lanes of every warp.
-template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class Load, class Store, class Alpha>
+// all 32 lanes of every warp. With SHARE the last rays are shared out within each warp
+// (share_rays), and fewer rays than lanes are spread over all warps, a few lanes of each; a
+// first-hit ray may then report any of its hits. Without it the visits are those of a
+// one-ray-at-a-time walk.
+template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, bool SHARE, class Load, class Store,
+          class Alpha>
 __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Load load,
-                                                 Store store, Alpha alpha, TraceCounters* ctr,
+                                                 Store store_hit, Alpha alpha, TraceCounters* ctr,
                                                  uint32_t* err, int refill_lanes,
                                                  int postpone_lanes) {
     const uint32_t lane = threadIdx.x & 31u;
     uint2 stack[kStackSize];
     auto st_ref = [&](int i) -> uint2& { return stack[i]; };
+    // the barycentrics are divided once, for the final hit
+    auto store = [&](uint32_t i, TraceState& s) {
+        if (s.best.geom != kNoInst) {
+            s.best.u = __fdiv_rn(s.best.u, s.det);
+            s.best.v = __fdiv_rn(s.best.v, s.det);
+        }
+        store_hit(i, s.best, (s.pre.k & kTriKey) >> kTriKeyShift);
+    };
     TraceState s;
+    s.best.geom = kNoInst;
+    s.aux = lane << 8;
     uint32_t ray = 0xFFFFFFFFu;
-    bool active = false, exhausted = false;
+    bool active = false, owns = false, pool_empty = false;
+    if (SHARE) {
+        const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+        const uint32_t lanes = (n + warps - 1u) / warps;
+        if (lanes < 32u) { // every warp has its rays at once, and the pool is empty
+            const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
+            if (lane < lanes && i < n) {
+                ray = i;
+                load(ray, s);
+                active = owns = true;
+            }
+            pool_empty = true;
+        }
+    }
     while (true) {
         __syncwarp();
-        const bool want = !active && !exhausted;
-        const uint32_t want_mask = __ballot_sync(0xFFFFFFFFu, want);
-        if (want_mask) {
-            const uint32_t leader = __ffs(want_mask) - 1u;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(want_mask));
-            base = __shfl_sync(0xFFFFFFFFu, base, leader);
-            if (want) {
-                ray = base + __popc(want_mask & ((1u << lane) - 1u));
-                if (ray < n) {
-                    load(ray, s);
-                    active = true;
-                } else {
-                    exhausted = true;
+        if (!SHARE || !pool_empty) {
+            bool exhausted = false;
+            const uint32_t want_mask = __ballot_sync(0xFFFFFFFFu, !active);
+            if (want_mask && !pool_empty) {
+                const uint32_t leader = __ffs(want_mask) - 1u;
+                uint32_t base = 0;
+                if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(want_mask));
+                base = __shfl_sync(0xFFFFFFFFu, base, leader);
+                if (!active) {
+                    const uint32_t i = base + __popc(want_mask & ((1u << lane) - 1u));
+                    if (i < n) {
+                        ray = i;
+                        load(ray, s);
+                        active = owns = true;
+                    } else {
+                        exhausted = true;
+                    }
                 }
+                pool_empty = __ballot_sync(0xFFFFFFFFu, exhausted) != 0u;
             }
         }
-        if (__ballot_sync(0xFFFFFFFFu, active) == 0u) break;
-        // once a lane found the pool empty, leaving the loop to refill gains nothing
-        const bool pool_empty = __ballot_sync(0xFFFFFFFFu, exhausted) != 0u;
+        if (SHARE && pool_empty) share_rays<MODE, TWO_LEVEL>(s, st_ref, ray, active, owns, store);
+        if (__ballot_sync(0xFFFFFFFFu, active) == 0u) {
+            if (!SHARE || __ballot_sync(0xFFFFFFFFu, owns) == 0u) break;
+            continue;
+        }
         if (!active) continue;
         const auto ray_alpha = [&](uint32_t g, uint32_t p, float u, float v) {
             return alpha(ray, g, p, u, v);
         };
-        if (trace_loop<MODE, COUNT, TWO_LEVEL>(s, st_ref, ctr, err, pool_empty, ray_alpha,
-                                                    refill_lanes, postpone_lanes)) {
-            store(ray, s.best, (s.pre.k & kTriKey) >> kTriKeyShift);
+        // until few lanes are busy and the pool can refill the others; with the pool empty a few
+        // steps between two shares, or to the end
+        s.aux &= 0xFFFFu;
+        if (trace_loop<MODE, COUNT, TWO_LEVEL>(
+                s, st_ref, ctr, err, ray_alpha, pool_empty ? (SHARE ? 33 : 0) : refill_lanes,
+                SHARE && pool_empty ? (kShareSteps - 1u) << 16 : 0u,
+                postpone_lanes)) {
             active = false;
+            if (!SHARE || !pool_empty) {
+                store(ray, s);
+                owns = false;
+                s.best.geom = kNoInst;
+            }
         }
     }
 }

@@ -45,15 +45,15 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         s.tris_base = sc.tris;
         s.tri_stride = sc.tri_stride;
         s.insts = sc.n_inst ? sc.inst : nullptr;
-        s.mask = mask;
         trace_init(s, f3(r.origin[0], r.origin[1], r.origin[2]),
-                   f3(r.direction[0], r.direction[1], r.direction[2]), r.tmin, r.tmax);
+                   f3(r.direction[0], r.direction[1], r.direction[2]), r.tmin, r.tmax,
+                   mask);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t) { hits[i] = to_hit(sc, h); };
     auto alpha = [&](uint32_t, uint32_t g, uint32_t p, float u, float v) {
         return alpha_discard(sc, g, p, u, v);
     };
-    trace_persistent<ANY ? kTraceAny : kTraceClosest, true, true>(n, fetch, load, store, alpha, &ctr, err, refill_lanes,
+    trace_persistent<ANY ? kTraceAny : kTraceClosest, true, true, false>(n, fetch, load, store, alpha, &ctr, err, refill_lanes,
                                       postpone_lanes);
     if (work_ctr) {
         atomicAdd(work_ctr + 0, (unsigned long long)ctr.nodes);
@@ -80,8 +80,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         s.tris_base = sc.tris;
         s.tri_stride = sc.tri_stride;
         s.insts = sc.n_inst ? sc.inst : nullptr;
-        s.mask = mask;
-        trace_init(s, o, d, tmin, tmax);
+        trace_init(s, o, d, tmin, tmax, mask);
     };
     auto store = [&](uint32_t i, const Hit& ht, uint32_t) {
         if (!texels) {
@@ -99,7 +98,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
     auto alpha = [&](uint32_t, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
-    trace_persistent<kTraceClosest, false, TWO_LEVEL>(w * h, fetch, load, store, alpha, nullptr, err,
+    trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(w * h, fetch, load, store, alpha, nullptr, err,
                                               refill_lanes, postpone_lanes);
 }
 

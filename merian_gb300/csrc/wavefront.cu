@@ -170,15 +170,14 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_trace_pixels(TickArg
         s.tris_base = c.tris;
         s.tri_stride = c.tri_stride;
         s.insts = c.insts;
-        s.mask = c.mask;
-        trace_init(s, o, d, tmin, tmax);
+        trace_init(s, o, d, tmin, tmax, c.mask);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t) { store_hit(t.w.hit, i, h); };
     auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(t.scenes[t.chunks[chunk_by_slot(t.chunks, nc, i)].scene], g,
                                       p, u, v);
     };
-    trace_persistent<kTraceClosest, false, TWO_LEVEL>(
+    trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(
         n, vertex_words(t, 0) + kCursor, load, store, alpha, nullptr, t.w.counters + 3,
         t.refill_lanes, t.postpone_lanes);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
@@ -404,9 +403,8 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
         s.tris_base = c.tris;
         s.tri_stride = c.tri_stride;
         s.insts = c.insts;
-        s.mask = c.mask;
         trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, shadow ? a.w : kRayTmax,
-                   shadow ? kRayAny : 0u);
+                   c.mask, shadow ? kRayAny : 0u);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t key) {
         if (i < n_rays) {
@@ -428,7 +426,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
     auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(t.scenes[chunk_of(i).scene], g, p, u, v);
     };
-    trace_persistent<kTraceMixed, COUNT, TWO_LEVEL>(
+    trace_persistent<kTraceMixed, COUNT, TWO_LEVEL, !COUNT>(
         n_rays + n_shadows, words + (parts == 2 ? kCursor2 : kCursor), load, store, alpha, &ctr,
         t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
     if (sort) {

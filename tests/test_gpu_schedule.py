@@ -125,3 +125,27 @@ def test_closest_and_shadow_rays_in_one_launch(gpu_ctx, kind):
     finally:
         gpu_ctx.set_profiling(0)
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("kind", ["room", "instanced", "alpha", "alpha-instanced"])
+def test_shared_rays(gpu_ctx, kind):
+    """A warp's last rays are shared out among its lanes, except in the counting traversal
+    (profiling level 2): the same bits, from a single ray to more rays than lanes."""
+    from merian_gb300 import scene as S
+    sc, (pos, target, fov) = _scenes()[kind]
+    if sc.env is None:
+        sc.env = np.ones((8, 16, 4), np.float32)
+    sid = gpu_ctx.upload(sc)
+    cam = S.look_at(pos, target, (0.0, 1.0, 0.0), fov, 1.0)
+    try:
+        for w, h, spp in [(1, 1, 1), (7, 1, 1), (71, 69, 1), (97, 50, 2), (401, 397, 1)]:
+            for nee in (False, True):
+                p, _ = S.render_params(w, h, spp, 8, nee=nee, frame=h)
+                a = gpu_ctx.render(sid, cam, p)
+                gpu_ctx.set_profiling(2)
+                b, _ = gpu_ctx.render(sid, cam, p, stats=True)
+                gpu_ctx.set_profiling(0)
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (w, h, nee)
+    finally:
+        gpu_ctx.set_profiling(0)
+        gpu_ctx.destroy_scene(sid)
