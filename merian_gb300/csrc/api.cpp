@@ -1590,7 +1590,7 @@ static int trace_common(gbpt_ctx* ctx, uint32_t scene, const gbpt_ray* rays, uin
         return GBPT_ERR_NOT_FOUND;
     }
     if (npr || tpr) GBPT_CUDA_CHECK(cudaMemsetAsync(ctx->d_misc, 0, 2 * sizeof(unsigned long long), ctx->stream));
-    rc = trace_rays(it->second, rays, n, mask, any_hit, hits, ctx->d_misc, ctx->stream,
+    rc = trace_rays(it->second, rays, n, mask, any_hit, hits, ctx->d_misc, npr || tpr, ctx->stream,
                     sched_of(ctx->tuning));
     if (rc) {
         set_error("gbpt_trace: launch failed");

@@ -801,10 +801,9 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
 // scene (nodes, tris, insts) and calls trace_init; store(i, hit, key) receives its result
 // and the material-sort key of the closest hit (0 on a miss);
 // alpha(i, geom, prim, u, v) is ray i's alpha test (true: skip the candidate). Must be called by
-// all 32 lanes of every warp. With SHARE the last rays are shared out within each warp
-// (share_rays), and fewer rays than lanes are spread over all warps, a few lanes of each; a
-// first-hit ray may then report any of its hits. Without it the visits are those of a
-// one-ray-at-a-time walk.
+// all 32 lanes of every warp. Fewer rays than lanes are spread over all warps, a few lanes of
+// each; with SHARE the last rays are shared out within each warp (share_rays), and a first-hit ray
+// may then report any of its hits. Without it the visits are those of a one-ray-at-a-time walk.
 template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, bool SHARE, class Load, class Store,
           class Alpha>
 __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Load load,
@@ -827,9 +826,9 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
     s.aux = lane << 8;
     uint32_t ray = 0xFFFFFFFFu;
     bool active = false, owns = false, pool_empty = false;
-    if (SHARE) {
+    if (!COUNT) {
         const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-        const uint32_t lanes = (n + warps - 1u) / warps;
+        const uint32_t lanes = n / warps + (n % warps != 0u ? 1u : 0u);
         if (lanes < 32u) { // every warp has its rays at once, and the pool is empty
             const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
             if (lane < lanes && i < n) {

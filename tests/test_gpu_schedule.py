@@ -149,3 +149,31 @@ def test_shared_rays(gpu_ctx, kind):
     finally:
         gpu_ctx.set_profiling(0)
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("kind", ["room", "instanced", "alpha", "alpha-instanced"])
+@pytest.mark.parametrize("any_hit", [False, True], ids=["closest", "any"])
+def test_ray_queries_equal_the_counting_traversal(gpu_ctx, kind, any_hit):
+    """gbpt_trace leaves out the code a scene does not need and spreads few rays over all warps;
+    gbpt_trace_counted runs the general traversal: the same hit records, first hits included."""
+    import torch
+    from merian_gb300 import _native as N
+    sc, (pos, target, fov) = _scenes()[kind]
+    side = 1.0 if sc.instances is None else (10.0 if kind == "instanced" else 4.0)
+    sid = gpu_ctx.upload(sc)
+    rng = np.random.default_rng(5)
+    try:
+        for n in (1, 31, 33, 4863, 4865, 200_001):
+            rays = np.zeros(n, N.RAY_DTYPE)
+            rays["origin"] = rng.uniform(0, side, (n, 3))
+            rays["direction"] = rng.normal(size=(n, 3))
+            rays["tmax"] = 1e7
+            r = torch.from_numpy(rays.view(np.float32).reshape(n, 8)).cuda()
+            h = [torch.full((n, 8), -1, dtype=torch.int32, device="cuda") for _ in range(2)]
+            torch.cuda.synchronize()
+            gpu_ctx.trace(sid, r.data_ptr(), n, h[0].data_ptr(), any_hit=any_hit)
+            gpu_ctx.trace(sid, r.data_ptr(), n, h[1].data_ptr(), any_hit=any_hit, counted=True)
+            gpu_ctx.synchronize()
+            assert torch.equal(h[0], h[1]), n
+    finally:
+        gpu_ctx.destroy_scene(sid)
