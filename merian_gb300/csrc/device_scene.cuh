@@ -762,7 +762,7 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     s.tris = shfl_ptr(s.tris, src);
     s.o = f3(f(s.o.x), f(s.o.y), f(s.o.z));
     s.inv = f3(f(s.inv.x), f(s.inv.y), f(s.inv.z));
-    s.tmin = f(s.tmin);
+    if (MODE != kTraceMixed) s.tmin = f(s.tmin); // bounce and shadow rays start at 0
     s.pre.Sx = f(s.pre.Sx);
     s.pre.Sy = f(s.pre.Sy);
     s.pre.Sz = f(s.pre.Sz);
