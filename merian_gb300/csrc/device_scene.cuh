@@ -352,7 +352,8 @@ GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tma
     s.wo = o;
     s.wd = d;
     s.tmin = tmin;
-    s.ngroup = make_uint2(0u, 0x80000000u);
+    // a span with a NaN end holds no hit (and would make every box test a hit)
+    s.ngroup = make_uint2(0u, tmin == tmin && tmax == tmax ? 0x80000000u : 0u);
     s.tgroup = make_uint2(0u, 0u);
     s.best.t = tmax;
     s.best.u = s.best.v = 0.0f;
@@ -419,14 +420,37 @@ template <int J> GBPT_DI float2 plane_t2(uint32_t w, uint64_t a2, uint64_t o2) {
     return r;
 }
 
-// Intersects the 8 children of node `ni`; returns the hit mask (inner children in bits 24..31 in
-// traversal order, triangles in bits 0..23) and the node's child / triangle bases and imask.
+// The order of a node's inner children: bit s of m to bit s ^ o, o the ray's inverted octant, so
+// that the highest bit is the child to visit first. One byte per (o, m), in shared memory.
+struct OctantOrder {
+    uint8_t bits[8 * 256];
+};
+GBPT_DI void octant_order_init(OctantOrder& t) {
+    for (uint32_t i = threadIdx.x; i < 8u * 256u; i += blockDim.x) {
+        uint32_t m = i & 255u;
+        const uint32_t o = i >> 8;
+        if (o & 1u) m = ((m >> 1) & 0x55u) | ((m << 1) & 0xAAu);
+        if (o & 2u) m = ((m >> 2) & 0x33u) | ((m << 2) & 0xCCu);
+        if (o & 4u) m = (m >> 4) | ((m << 4) & 0xF0u);
+        t.bits[i] = (uint8_t)m;
+    }
+    __syncthreads();
+}
+
+// Bound by the ALU pipe (byte permutes, minima and maxima, at half the FMA pipe's rate), so what can
+// go elsewhere does: hits are collected from the signs of differences (FMA pipe) instead of
+// compares and shifted meta bytes, the visiting order comes from a table in shared memory, and only
+// the leaves that are hit (one in six nodes has any) look at their meta bytes: 1080p soup frame
+// 251.7 instead of 258.2 ms.
+// Intersects the 8 children of node `ni`. ngroup receives the child base and the inner children
+// hit in visiting order in bits 24..31, the node's imask in bits 0..7; tgroup the triangle base
+// and the hit leaves' triangles in bits 0..23.
 // The quantised planes are dequantised with a per-axis slack of 2^-20 of the plane distance
 // magnitude (plus 2^-8 of a quantisation step for the biased planes), so rounding never loses a
 // child the exact box would keep.
-template <bool COUNT, bool PAIRED = GBPT_BOX_FMA2 != 0>
-GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& child_base,
-                                uint32_t& tri_base, uint32_t& imask, TraceCounters* ctr) {
+template <bool COUNT, bool PAIRED>
+GBPT_DI void intersect_node(const TraceState& s, uint32_t ni, const OctantOrder& order,
+                            uint2& ngroup, uint2& tgroup, TraceCounters* ctr) {
     if (COUNT) ctr->nodes++;
     const uint4 n0 = __ldg(&s.nodes[5 * ni + 0]);
     const uint4 n1 = __ldg(&s.nodes[5 * ni + 1]);
@@ -455,23 +479,20 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
     const float foy = __fmaf_rn(-kPlaneBias, aiy, __fadd_rn(aoy, ey));
     const float noz = __fmaf_rn(-kPlaneBias, aiz, __fsub_rn(aoz, ez));
     const float foz = __fmaf_rn(-kPlaneBias, aiz, __fadd_rn(aoz, ez));
-    imask = n0.w >> 24;
-    child_base = n1.x;
-    tri_base = n1.y;
+    const uint32_t imask = n0.w >> 24;
 
     // the direction's signs from the octant (negative axis a: bit a of oct_inv clear)
     const uint32_t oct_inv = s.pre.oct_inv();
-    const uint32_t oct_inv4 = oct_inv * 0x01010101u;
     const bool negx = (oct_inv & 1u) == 0u, negy = (oct_inv & 2u) == 0u;
     const bool negz = (oct_inv & 4u) == 0u;
-    uint32_t hitmask = 0;
+    // the children missed, the first child in the highest bit: the sign of cmax - cmin is set
+    // exactly when cmin <= cmax is false (no NaN gets here: trace_init ends such rays)
+    uint32_t miss = 0;
+    auto add = [&](float cmin, float cmax) {
+        miss = __funnelshift_l(__float_as_uint(__fsub_rn(cmax, cmin)), miss, 1);
+    };
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-        const uint32_t meta4 = half ? n1.w : n1.z;
-        const uint32_t is_inner4 = (meta4 & (meta4 << 1)) & 0x10101010u;
-        const uint32_t inner_mask4 = (is_inner4 >> 4) * 0xFFu;
-        const uint32_t bit_index4 = (meta4 ^ (oct_inv4 & inner_mask4)) & 0x1F1F1F1Fu;
-        const uint32_t child_bits4 = (meta4 >> 5) & 0x07070707u;
         const uint32_t qlx = half ? n2.y : n2.x, qly = half ? n2.w : n2.z;
         const uint32_t qlz = half ? n3.y : n3.x, qhx = half ? n3.w : n3.z;
         const uint32_t qhy = half ? n4.y : n4.x, qhz = half ? n4.w : n4.z;
@@ -493,18 +514,14 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
                 const float cmax0 = fminf(fminf(tfx.x, tfy.x), fminf(tfz.x, s.best.t));
                 const float cmin1 = fmaxf(fmaxf(tnx.y, tny.y), fmaxf(tnz.y, s.tmin));
                 const float cmax1 = fminf(fminf(tfx.y, tfy.y), fminf(tfz.y, s.best.t));
-                constexpr uint32_t sh0 = 8u * j, sh1 = 8u * (j + 1);
-                if (cmin0 <= cmax0)
-                    hitmask |= ((child_bits4 >> sh0) & 7u) << ((bit_index4 >> sh0) & 31u);
-                if (cmin1 <= cmax1)
-                    hitmask |= ((child_bits4 >> sh1) & 7u) << ((bit_index4 >> sh1) & 31u);
+                add(cmin0, cmax0);
+                add(cmin1, cmax1);
             };
             pair(std::integral_constant<int, 0>{});
             pair(std::integral_constant<int, 2>{});
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const uint32_t sh = 8u * j;
                 const float tnx = __fmaf_rn(qplane(nqx, j), aix, nox);
                 const float tny = __fmaf_rn(qplane(nqy, j), aiy, noy);
                 const float tnz = __fmaf_rn(qplane(nqz, j), aiz, noz);
@@ -513,12 +530,23 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
                 const float tfz = __fmaf_rn(qplane(fqz, j), aiz, foz);
                 const float cmin = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, s.tmin));
                 const float cmax = fminf(fminf(tfx, tfy), fminf(tfz, s.best.t));
-                if (cmin <= cmax)
-                    hitmask |= ((child_bits4 >> sh) & 7u) << ((bit_index4 >> sh) & 31u);
+                add(cmin, cmax);
             }
         }
     }
-    return hitmask;
+    const uint32_t hits = (__brev(miss) >> 24) ^ 0xFFu; // by child
+    const uint32_t inner = hits & imask;
+    const uint32_t first = order.bits[(s.pre.k & 0x700u) | inner];
+    ngroup = make_uint2(n1.x, (first << 24) | imask);
+    // the leaves' triangles, from their meta bytes: unary count << 5 | first triangle
+    uint32_t leaves = hits & ~imask, tri = 0u;
+    while (leaves != 0u) {
+        const uint32_t j = __ffs(leaves) - 1u;
+        leaves &= leaves - 1u;
+        const uint32_t meta = __byte_perm(n1.z, n1.w, j) & 0xFFu;
+        tri |= (meta >> 5) << (meta & 31u);
+    }
+    tgroup = make_uint2(n1.y, tri);
 }
 
 // Runs the traversal of the ray in s until it is finished (returns true; result in s.best, geom
@@ -527,10 +555,12 @@ GBPT_DI uint32_t intersect_node(const TraceState& s, uint32_t ni, uint32_t& chil
 // and finishes the ray with what it found.
 // `alpha(geom, prim, u, v)` decides the candidate hits of non-opaque triangles (true: skip).
 template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class StackRef, class Alpha>
-GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32_t* err,
+GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, const OctantOrder& order,
+                        TraceCounters* ctr, uint32_t* err,
                         const Alpha& alpha, int min_lanes, uint32_t step_mask,
                         int postpone_lanes) {
     while (true) {
+        const bool any = MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u);
         if (s.ngroup.y > 0x00FFFFFFu) {
             const uint32_t hits = s.ngroup.y;
             const uint32_t bit = 31u - __clz(hits & 0xFF000000u);
@@ -549,14 +579,11 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
             }
             const uint32_t slot = (bit - 24u) ^ s.pre.oct_inv();
             const uint32_t ni = s.ngroup.x + __popc((hits & 0xFFu) & ((1u << slot) - 1u));
-            uint32_t cb, tb, im;
             if (COUNT) count_step(ctr->node_steps, ctr->node_lanes);
             // the paired planes hold more registers: first-hit traversal, which keeps fewer,
             // measured faster with the scalar ones
-            const uint32_t hm =
-                intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(s, ni, cb, tb, im, ctr);
-            s.ngroup = make_uint2(cb, (hm & 0xFF000000u) | im);
-            s.tgroup = make_uint2(tb, hm & 0x00FFFFFFu);
+            intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(s, ni, order, s.ngroup,
+                                                                           s.tgroup, ctr);
         } else {
             // a postponed triangle group (or the rest of a top-level instance group) came off
             // the stack
@@ -566,7 +593,6 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, TraceCounters* ctr, uint32
         bool done_any = false;
         // only groups followed by node work are postponed (a group popped back is tested), and
         // never those of a first-hit query, which any of its triangles may end
-        const bool any = MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u);
         const bool may_postpone = !any && s.ngroup.y > 0x00FFFFFFu;
         while (s.tgroup.y != 0u) {
             if (may_postpone && s.sp() < kStackSize && __popc(__activemask()) < postpone_lanes) {
@@ -811,6 +837,8 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
                                                  uint32_t* err, int refill_lanes,
                                                  int postpone_lanes) {
     const uint32_t lane = threadIdx.x & 31u;
+    __shared__ OctantOrder order;
+    octant_order_init(order);
     uint2 stack[kStackSize];
     auto st_ref = [&](int i) -> uint2& { return stack[i]; };
     // the barycentrics are divided once, for the final hit
@@ -875,7 +903,7 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
         // steps between two shares, or to the end
         s.aux &= 0xFFFFu;
         if (trace_loop<MODE, COUNT, TWO_LEVEL>(
-                s, st_ref, ctr, err, ray_alpha, pool_empty ? (SHARE ? 33 : 0) : refill_lanes,
+                s, st_ref, order, ctr, err, ray_alpha, pool_empty ? (SHARE ? 33 : 0) : refill_lanes,
                 SHARE && pool_empty ? (kShareSteps - 1u) << 16 : 0u,
                 postpone_lanes)) {
             active = false;

@@ -177,3 +177,48 @@ def test_ray_queries_equal_the_counting_traversal(gpu_ctx, kind, any_hit):
             assert torch.equal(h[0], h[1]), n
     finally:
         gpu_ctx.destroy_scene(sid)
+
+
+def test_rays_with_special_values(gpu_ctx):
+    """Zero directions components, infinite spans, spans with a NaN end, reversed and empty spans:
+    closest and first hits as the FP32 oracle's (a NaN end: no hit)."""
+    import torch
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    from oracle import binding as O
+    sc = S.soup(n_triangles=5_000, n_geometries=16, env_size=None)
+    osc = O.OracleScene(sc)
+    sid = gpu_ctx.upload(sc)
+    rng = np.random.default_rng(8)
+    n = 4096
+    rays = np.zeros(n, N.RAY_DTYPE)
+    rays["origin"] = rng.uniform(-0.1, 1.1, (n, 3))
+    rays["direction"] = rng.normal(size=(n, 3))
+    rays["direction"][rng.uniform(size=(n, 3)) < 0.1] = 0.0
+    rays["direction"][(rays["direction"] == 0).all(1)] = (0, 0, 1)
+    kind = rng.integers(0, 5, n)
+    rays["tmax"] = np.select([kind == 0, kind == 1, kind == 2], [np.inf, 0.3, -1.0], 1e7)
+    rays["tmin"] = np.where(kind == 3, -0.5, 0.0)
+    nan = kind == 4
+    rays["tmin"][nan & (np.arange(n) % 2 == 0)] = np.nan
+    rays["tmax"][nan & (np.arange(n) % 2 == 1)] = np.nan
+    try:
+        o, _, _ = osc.trace_rays(np.ascontiguousarray(rays[~nan]), fp64=False,
+                                 hit_dtype=N.HIT_DTYPE)
+        r = torch.from_numpy(rays.view(np.float32).reshape(n, 8)).cuda()
+        h = torch.zeros((n, 8), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        for any_hit in (False, True):
+            gpu_ctx.trace(sid, r.data_ptr(), n, h.data_ptr(), any_hit=any_hit)
+            gpu_ctx.synchronize()
+            g = np.frombuffer(h.cpu().numpy().tobytes(), N.HIT_DTYPE)
+            assert (g["geometry_index"][nan] == 0xFFFFFFFF).all()
+            g = g[~nan]
+            if any_hit:
+                assert np.array_equal(g["geometry_index"] == 0xFFFFFFFF,
+                                      o["geometry_index"] == 0xFFFFFFFF)
+            else:
+                for f in ("geometry_index", "primitive_id", "t"):
+                    assert np.array_equal(g[f].view(np.uint32), o[f].view(np.uint32)), f
+    finally:
+        gpu_ctx.destroy_scene(sid)
