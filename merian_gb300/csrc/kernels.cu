@@ -39,7 +39,7 @@ GBPT_DI gbpt_hit to_hit(const DevScene& sc, const Hit& h) {
 // soup take 0.85 instead of 1.19 ms, 250,000 occlusion rays in the tessellated room 0.15 instead
 // of 0.33.
 template <bool ANY, bool COUNT, bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, kTraceBlocksPerSM)
+__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     k_trace_rays(DevScene sc, const gbpt_ray* rays, uint32_t n, uint32_t mask, gbpt_hit* hits,
                  unsigned long long* work_ctr, uint32_t* fetch, uint32_t* err, int refill_lanes,
                  int postpone_lanes) {
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(128, kTraceBlocksPerSM)
 // its longest ray was done: the 1920x1080 G-buffer of the instanced scene took 2.43 instead of
 // 0.94 ms.
 template <bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, kTraceBlocksPerSM)
+__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     k_trace_primary(DevScene sc, CamGPU cam, uint32_t w, uint32_t h, uint32_t mask, gbpt_hit* hits,
                     gbpt_gbuffer_texel* texels, uint32_t* fetch, uint32_t* err, int refill_lanes,
                     int postpone_lanes) {

@@ -168,7 +168,7 @@ GBPT_DI const ChunkGPU& slot_ray(const TickArgs& t, uint32_t nc, uint32_t q, flo
 // instanced 1280x720 frame 1.80 instead of 0.36 ms, of the 640x360 soup frame 0.54 instead of
 // 0.21 ms; the frames 8.84 instead of 7.47 and 12.42 instead of 12.11 ms).
 template <bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, kTraceBlocksPerSM) k_trace_pixels(TickArgs t) {
+__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL)) k_trace_pixels(TickArgs t) {
     wait_for_predecessor();
     const uint32_t n = t.hdr->n_pix, nc = t.hdr->n_chunks;
     auto load = [&](uint32_t i, TraceState& s) {
@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
 // 640x360 soup frame 8.6 instead of 9.4; the clears of the counters, now one per tick instead of
 // four per vertex, included).
 template <bool COUNT, bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, kTraceBlocksPerSM)
+__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     k_trace(TickArgs t, int k, int qi, int parts, unsigned long long* work_ctr, int sort) {
     wait_for_predecessor();
     uint32_t* words = vertex_words(t, k);
@@ -871,7 +871,8 @@ uint32_t sorted_vertices(const TickPlan& tp, int kinds) {
 struct Grids {
     int grid;    // grid-stride kernels without a register budget (finalize, material sort)
     int trace;   // persistent traversal: the blocks resident at once
-    int trace_c;
+    int trace2;  // ... of the two-level variants
+    int trace_c; // ... of the counting ones
     int primary; // k_primary, k_shade_primary, k_shade: their resident blocks
     int shade_p;
     int shade;
@@ -879,9 +880,10 @@ struct Grids {
 Grids launch_grids() {
     Grids g;
     g.grid = num_sms() * 8;
-    // the two-level and alpha variants have the same launch bounds, hence the same residency
+    // the alpha variants have the same launch bounds, hence the same residency
     g.trace = persistent_grid(k_trace<false, false, false>);
-    g.trace_c = persistent_grid(k_trace<true, false, false>);
+    g.trace2 = persistent_grid(k_trace<false, true, false>);
+    g.trace_c = persistent_grid(k_trace<true, true, false>);
     g.primary = persistent_grid(k_primary);
     g.shade_p = persistent_grid(k_shade_primary);
     g.shade = persistent_grid(k_shade);
@@ -907,7 +909,7 @@ void launch(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... arg
 
 void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k, int qi, int parts,
                   unsigned long long* work_ctr, bool sort, cudaStream_t st) {
-    const int gr = work_ctr ? g.trace_c : g.trace;
+    const int gr = work_ctr ? g.trace_c : tp.two_level ? g.trace2 : g.trace;
     const int so = sort ? 1 : 0;
     auto go = [&](auto kernel) { launch(kernel, gr, 128, st, ta, k, qi, parts, work_ctr, so); };
     switch ((work_ctr ? 4 : 0) | (tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
@@ -948,7 +950,10 @@ uint64_t enqueue_tick(const TickArgs& ta, const TickPlan& tp, const Grids& g, cu
         cudaMemsetAsync(ctr + kSortWord, 0, (tp.sorted + 1) * 8 * sizeof(uint32_t), st);
     const int pgrid = (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.primary);
     int ev = prof->begin(st, 3);
-    launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.trace), st);
+    launch_trace_pixels(ta, tp,
+                        (int)std::min<uint64_t>((pix + 127) / 128,
+                                                (uint64_t)(tp.two_level ? g.trace2 : g.trace)),
+                        st);
     launch(k_primary, pgrid, 128, st, ta, tp.sorted >= 1 ? 1 : 0);
     prof->end(st, ev);
     nl += 2;
@@ -1140,6 +1145,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     if (e.sched.blocks_per_sm > 0) {
         const int cap = (int)e.sched.blocks_per_sm * num_sms();
         grids.trace = std::min(grids.trace, cap);
+        grids.trace2 = std::min(grids.trace2, cap);
         grids.trace_c = std::min(grids.trace_c, cap);
     }
     uint64_t nl = 0;
