@@ -332,6 +332,31 @@ struct TraceState {
     GBPT_DI void clear_sp() { pre.k &= 0x00FFFFFFu; }
 };
 
+// Where a launch's rays find their scene: in each ray's state (requests of several scenes share
+// ticks), or, when all rays are of one scene, in the kernel's arguments. The latter saves the
+// two-level state five registers (instanced 1280x720 frame 4.09 instead of 4.25 ms; its G-buffer
+// 0.86 instead of 0.90) and the ray queries' two (a million closest hits 0.81 instead of 0.86);
+// the single-level wavefront is no faster with it (1080p soup frame 253.4 against 251.8 ms).
+struct SceneRef {
+    const uint4* nodes;
+    const float4* tris;
+    const float4* insts;
+    uint32_t tri_stride;
+};
+struct RayScene {
+    static constexpr bool kPerRay = true;
+    GBPT_DI const uint4* nodes(const TraceState& s) const { return s.nodes; }
+    GBPT_DI const float4* tris(const TraceState& s) const { return s.tris; }
+    GBPT_DI const float4* insts(const TraceState& s) const { return s.insts; }
+};
+struct OneScene {
+    static constexpr bool kPerRay = false;
+    SceneRef ref;
+    GBPT_DI const uint4* nodes(const TraceState&) const { return ref.nodes; }
+    GBPT_DI const float4* tris(const TraceState& s) const { return s.tris; }
+    GBPT_DI const float4* insts(const TraceState&) const { return ref.insts; }
+};
+
 GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
     s.o = o;
     s.d = d;
@@ -362,8 +387,8 @@ GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tma
     s.inst_sp = -1;
 }
 
-GBPT_DI void enter_instance(TraceState& s, uint32_t ii) {
-    const float4* r = s.insts + 7ull * ii;
+GBPT_DI void enter_instance(TraceState& s, const float4* insts, uint32_t ii) {
+    const float4* r = insts + 7ull * ii;
     const float4 w0 = __ldg(r + 3), w1 = __ldg(r + 4), w2 = __ldg(r + 5);
     set_ray(s, xform_point(w0, w1, w2, s.wo), xform_vector(w0, w1, w2, s.wd));
     s.inst = ii;
@@ -449,14 +474,14 @@ GBPT_DI void octant_order_init(OctantOrder& t) {
 // magnitude (plus 2^-8 of a quantisation step for the biased planes), so rounding never loses a
 // child the exact box would keep.
 template <bool COUNT, bool PAIRED>
-GBPT_DI void intersect_node(const TraceState& s, uint32_t ni, const OctantOrder& order,
+GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni, const OctantOrder& order,
                             uint2& ngroup, uint2& tgroup, TraceCounters* ctr) {
     if (COUNT) ctr->nodes++;
-    const uint4 n0 = __ldg(&s.nodes[5 * ni + 0]);
-    const uint4 n1 = __ldg(&s.nodes[5 * ni + 1]);
-    const uint4 n2 = __ldg(&s.nodes[5 * ni + 2]);
-    const uint4 n3 = __ldg(&s.nodes[5 * ni + 3]);
-    const uint4 n4 = __ldg(&s.nodes[5 * ni + 4]);
+    const uint4 n0 = __ldg(&nodes[5 * ni + 0]);
+    const uint4 n1 = __ldg(&nodes[5 * ni + 1]);
+    const uint4 n2 = __ldg(&nodes[5 * ni + 2]);
+    const uint4 n3 = __ldg(&nodes[5 * ni + 3]);
+    const uint4 n4 = __ldg(&nodes[5 * ni + 4]);
     const float kErr = 1.0f / 1048576.0f;
     const float kBiasErr = GBPT_BOX_BIAS ? 1.0f / 256.0f : 0.0f;
     // every operation rounded once in a fixed order (no contraction choices left to the
@@ -554,8 +579,8 @@ GBPT_DI void intersect_node(const TraceState& s, uint32_t ni, const OctantOrder&
 // lanes (returns false; s keeps the state). `st(i)` is stack entry i. A stack overflow raises *err
 // and finishes the ray with what it found.
 // `alpha(geom, prim, u, v)` decides the candidate hits of non-opaque triangles (true: skip).
-template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class StackRef, class Alpha>
-GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, const OctantOrder& order,
+template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class Scene, class StackRef, class Alpha>
+GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const OctantOrder& order,
                         TraceCounters* ctr, uint32_t* err,
                         const Alpha& alpha, int min_lanes, uint32_t step_mask,
                         int postpone_lanes) {
@@ -582,8 +607,8 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, const OctantOrder& order,
             if (COUNT) count_step(ctr->node_steps, ctr->node_lanes);
             // the paired planes hold more registers: first-hit traversal, which keeps fewer,
             // measured faster with the scalar ones
-            intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(s, ni, order, s.ngroup,
-                                                                           s.tgroup, ctr);
+            intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(
+                s, scene.nodes(s), ni, order, s.ngroup, s.tgroup, ctr);
         } else {
             // a postponed triangle group (or the rest of a top-level instance group) came off
             // the stack
@@ -604,9 +629,9 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, const OctantOrder& order,
             const uint32_t b = __ffs(s.tgroup.y) - 1u;
             s.tgroup.y &= s.tgroup.y - 1u;
             const uint32_t ti = s.tgroup.x + b;
-            if (TWO_LEVEL && s.insts != nullptr && s.inst == kNoInst) {
+            if (TWO_LEVEL && scene.insts(s) != nullptr && s.inst == kNoInst) {
                 // a top-level leaf: an instance (record: instance index, mask in the flag word)
-                const uint32_t fl = __float_as_uint(__ldg(&s.tris[3 * ti + 2]).w);
+                const uint32_t fl = __float_as_uint(__ldg(&scene.tris(s)[3 * ti + 2]).w);
                 if ((fl & s.pre.mask()) == 0u) continue;
                 if (s.sp() + 2 > kStackSize) {
                     atomicOr(err, 1u);
@@ -622,10 +647,10 @@ GBPT_DI bool trace_loop(TraceState& s, StackRef&& st, const OctantOrder& order,
                     s.push_sp();
                 }
                 s.tgroup.y = 0u;
-                enter_instance(s, __float_as_uint(__ldg(&s.tris[3 * ti]).w));
+                enter_instance(s, scene.insts(s), __float_as_uint(__ldg(&scene.tris(s)[3 * ti]).w));
                 break;
             }
-            const float4* rec = s.tris + 3 * ti;
+            const float4* rec = scene.tris(s) + 3 * ti;
             const float4 r0 = __ldg(rec + 0);
             const float4 r1 = __ldg(rec + 1);
             const float4 r2 = __ldg(rec + 2);
@@ -720,7 +745,7 @@ GBPT_DI bool hit_before(float t, uint32_t geom, uint32_t prim, uint32_t inst, co
 // frame, 1.81 / 1.79 / 1.79 / 1.86 on the pixel list, 260.6 / 260.8 / 261.5 (2 / 4 / 8) on the 1080p
 // soup.
 constexpr uint32_t kShareSteps = 2; // a power of two
-template <TraceMode MODE, bool TWO_LEVEL, class StackRef, class Store>
+template <TraceMode MODE, bool TWO_LEVEL, bool PER_RAY, class StackRef, class Store>
 GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& active, bool& owns,
                         const Store& store) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -784,7 +809,7 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     const uint32_t src = take ? nth_bit(m_donor, r) : lane;
     auto f = [&](float x) { return __shfl_sync(0xFFFFFFFFu, x, src); };
     auto w = [&](uint32_t x) { return __shfl_sync(0xFFFFFFFFu, x, src); };
-    s.nodes = shfl_ptr(s.nodes, src);
+    if (PER_RAY) s.nodes = shfl_ptr(s.nodes, src);
     s.tris = shfl_ptr(s.tris, src);
     s.o = f3(f(s.o.x), f(s.o.y), f(s.o.z));
     s.inv = f3(f(s.inv.x), f(s.inv.y), f(s.inv.z));
@@ -802,9 +827,11 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     e.y = w(e.y);
     bool restart = false;
     if (TWO_LEVEL) {
-        s.tris_base = shfl_ptr(s.tris_base, src);
-        s.tri_stride = w(s.tri_stride);
-        s.insts = shfl_ptr(s.insts, src);
+        if (PER_RAY) {
+            s.tris_base = shfl_ptr(s.tris_base, src);
+            s.tri_stride = w(s.tri_stride);
+            s.insts = shfl_ptr(s.insts, src);
+        }
         s.wo = f3(f(s.wo.x), f(s.wo.y), f(s.wo.z));
         s.wd = f3(f(s.wd.x), f(s.wd.y), f(s.wd.z));
         s.inst = w(s.inst);
@@ -823,16 +850,17 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
 }
 
 // Runs the traversal of every ray i < n with persistent warps that pull ray indices from *fetch
-// (zero before the launch; one atomic per warp for all idle lanes). load(i, state) sets ray i's
-// scene (nodes, tris, insts) and calls trace_init; store(i, hit, key) receives its result
+// (zero before the launch; one atomic per warp for all idle lanes). load(i, state) calls
+// trace_init and, when `scene` is per ray, sets ray i's scene (nodes, tris, insts) before; store(i, hit, key) receives its result
 // and the material-sort key of the closest hit (0 on a miss);
 // alpha(i, geom, prim, u, v) is ray i's alpha test (true: skip the candidate). Must be called by
 // all 32 lanes of every warp. Fewer rays than lanes are spread over all warps, a few lanes of
 // each; with SHARE the last rays are shared out within each warp (share_rays), and a first-hit ray
 // may then report any of its hits. Without it the visits are those of a one-ray-at-a-time walk.
-template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, bool SHARE, class Load, class Store,
-          class Alpha>
-__device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Load load,
+template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, bool SHARE, class Scene, class Load,
+          class Store, class Alpha>
+__device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n, uint32_t* fetch,
+                                                 Load load,
                                                  Store store_hit, Alpha alpha, TraceCounters* ctr,
                                                  uint32_t* err, int refill_lanes,
                                                  int postpone_lanes) {
@@ -890,7 +918,7 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
                 pool_empty = __ballot_sync(0xFFFFFFFFu, exhausted) != 0u;
             }
         }
-        if (SHARE && pool_empty) share_rays<MODE, TWO_LEVEL>(s, st_ref, ray, active, owns, store);
+        if (SHARE && pool_empty) share_rays<MODE, TWO_LEVEL, Scene::kPerRay>(s, st_ref, ray, active, owns, store);
         if (__ballot_sync(0xFFFFFFFFu, active) == 0u) {
             if (!SHARE || __ballot_sync(0xFFFFFFFFu, owns) == 0u) break;
             continue;
@@ -903,7 +931,7 @@ __device__ __forceinline__ void trace_persistent(uint32_t n, uint32_t* fetch, Lo
         // steps between two shares, or to the end
         s.aux &= 0xFFFFu;
         if (trace_loop<MODE, COUNT, TWO_LEVEL>(
-                s, st_ref, order, ctr, err, ray_alpha, pool_empty ? (SHARE ? 33 : 0) : refill_lanes,
+                s, scene, st_ref, order, ctr, err, ray_alpha, pool_empty ? (SHARE ? 33 : 0) : refill_lanes,
                 SHARE && pool_empty ? (kShareSteps - 1u) << 16 : 0u,
                 postpone_lanes)) {
             active = false;

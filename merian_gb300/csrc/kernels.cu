@@ -32,6 +32,10 @@ GBPT_DI gbpt_hit to_hit(const DevScene& sc, const Hit& h) {
     return out;
 }
 
+GBPT_DI OneScene one_scene(const DevScene& sc) {
+    return OneScene{{sc.nodes, sc.tris, sc.n_inst ? sc.inst : nullptr, sc.tri_stride}};
+}
+
 // The caller's rays through the persistent traversal (the closest hit or, with ANY, any hit).
 // Bound like the wavefront's traversal by issue slots. A first-hit ray is never shared among
 // lanes: the hit it reports is the first of its own walk. Scenes without instances or alpha tests,
@@ -46,10 +50,8 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     TraceCounters ctr{0, 0, 0, 0, 0, 0};
     auto load = [&](uint32_t i, TraceState& s) {
         const gbpt_ray r = rays[i];
-        s.nodes = sc.nodes;
         s.tris_base = sc.tris;
         s.tri_stride = sc.tri_stride;
-        s.insts = sc.n_inst ? sc.inst : nullptr;
         trace_init(s, f3(r.origin[0], r.origin[1], r.origin[2]),
                    f3(r.direction[0], r.direction[1], r.direction[2]), r.tmin, r.tmax, mask);
     };
@@ -58,7 +60,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
     trace_persistent<ANY ? kTraceAny : kTraceClosest, COUNT, TWO_LEVEL, !ANY && !COUNT>(
-        n, fetch, load, store, alpha, &ctr, err, refill_lanes, postpone_lanes);
+        one_scene(sc), n, fetch, load, store, alpha, &ctr, err, refill_lanes, postpone_lanes);
     if (COUNT) {
         atomicAdd(work_ctr + 0, (unsigned long long)ctr.nodes);
         atomicAdd(work_ctr + 1, (unsigned long long)ctr.tris);
@@ -80,10 +82,8 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
         float3 o, d;
         float tmin, tmax;
         camera_ray(cam, i % w, i / w, w, h, o, d, tmin, tmax);
-        s.nodes = sc.nodes;
         s.tris_base = sc.tris;
         s.tri_stride = sc.tri_stride;
-        s.insts = sc.n_inst ? sc.inst : nullptr;
         trace_init(s, o, d, tmin, tmax, mask);
     };
     auto store = [&](uint32_t i, const Hit& ht, uint32_t) {
@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     auto alpha = [&](uint32_t, uint32_t g, uint32_t p, float u, float v) {
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
-    trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(w * h, fetch, load, store, alpha, nullptr, err,
-                                              refill_lanes, postpone_lanes);
+    trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(
+        one_scene(sc), w * h, fetch, load, store, alpha, nullptr, err, refill_lanes,
+        postpone_lanes);
 }
 
 GBPT_DI uint32_t pack_half2_rn(float lo, float hi) {

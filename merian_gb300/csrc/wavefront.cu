@@ -167,18 +167,24 @@ GBPT_DI const ChunkGPU& slot_ray(const TickArgs& t, uint32_t nc, uint32_t q, flo
 // and the traversal spilled into the shading's registers (primary hits and shading points of the
 // instanced 1280x720 frame 1.80 instead of 0.36 ms, of the 640x360 soup frame 0.54 instead of
 // 0.21 ms; the frames 8.84 instead of 7.47 and 12.42 instead of 12.11 ms).
-template <bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL)) k_trace_pixels(TickArgs t) {
+template <bool TWO_LEVEL, bool ALPHA, class Scene>
+__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
+    k_trace_pixels(TickArgs t, Scene scene) {
     wait_for_predecessor();
     const uint32_t n = t.hdr->n_pix, nc = t.hdr->n_chunks;
     auto load = [&](uint32_t i, TraceState& s) {
         float3 o, d;
         float tmin, tmax;
         const ChunkGPU& c = slot_ray(t, nc, i, o, d, tmin, tmax);
-        s.nodes = c.nodes;
-        s.tris_base = c.tris;
-        s.tri_stride = c.tri_stride;
-        s.insts = c.insts;
+        if constexpr (Scene::kPerRay) {
+            s.nodes = c.nodes;
+            s.tris_base = c.tris;
+            s.tri_stride = c.tri_stride;
+            s.insts = c.insts;
+        } else {
+            s.tris_base = scene.ref.tris;
+            s.tri_stride = scene.ref.tri_stride;
+        }
         trace_init(s, o, d, tmin, tmax, c.mask);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t) { store_hit(t.w.hit, i, h); };
@@ -187,7 +193,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL)) k_trace_pixels(T
                                       p, u, v);
     };
     trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(
-        n, vertex_words(t, 0) + kCursor, load, store, alpha, nullptr, t.w.counters + 3,
+        scene, n, vertex_words(t, 0) + kCursor, load, store, alpha, nullptr, t.w.counters + 3,
         t.refill_lanes, t.postpone_lanes);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
 }
@@ -385,9 +391,10 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
 // 0.28 instead of 0.41 ms, the instanced 1280x720 frame of path length 16 5.6 instead of 7.6, the
 // 640x360 soup frame 8.6 instead of 9.4; the clears of the counters, now one per tick instead of
 // four per vertex, included).
-template <bool COUNT, bool TWO_LEVEL, bool ALPHA>
+template <bool COUNT, bool TWO_LEVEL, bool ALPHA, class Scene>
 __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
-    k_trace(TickArgs t, int k, int qi, int parts, unsigned long long* work_ctr, int sort) {
+    k_trace(TickArgs t, Scene scene, int k, int qi, int parts, unsigned long long* work_ctr,
+            int sort) {
     wait_for_predecessor();
     uint32_t* words = vertex_words(t, k);
     const uint32_t n_rays = (parts & 1) ? words[kRaysOut] : 0u;
@@ -411,10 +418,15 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
         const float4 a = e[0], b = e[1];
         const uint32_t tag = shadow ? __ldg(&t.w.s_path[i - n_rays]) : __float_as_uint(b.w);
         const ChunkGPU& c = t.chunks[tag >> kPathBits];
-        s.nodes = c.nodes;
-        s.tris_base = c.tris;
-        s.tri_stride = c.tri_stride;
-        s.insts = c.insts;
+        if constexpr (Scene::kPerRay) {
+            s.nodes = c.nodes;
+            s.tris_base = c.tris;
+            s.tri_stride = c.tri_stride;
+            s.insts = c.insts;
+        } else {
+            s.tris_base = scene.ref.tris;
+            s.tri_stride = scene.ref.tri_stride;
+        }
         trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, shadow ? a.w : kRayTmax,
                    c.mask, shadow ? kRayAny : 0u);
     };
@@ -439,7 +451,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
         return ALPHA && alpha_discard(t.scenes[chunk_of(i).scene], g, p, u, v);
     };
     trace_persistent<kTraceMixed, COUNT, TWO_LEVEL, !COUNT>(
-        n_rays + n_shadows, words + (parts == 2 ? kCursor2 : kCursor), load, store, alpha, &ctr,
+        scene, n_rays + n_shadows, words + (parts == 2 ? kCursor2 : kCursor), load, store, alpha, &ctr,
         t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
     if (sort) {
         __syncthreads();
@@ -849,6 +861,10 @@ struct TickPlan {
     bool nee;
     bool two_level; // some chunk's scene is instanced: the two-level traversal variants
     bool alpha;     // some chunk's scene has alpha-tested geometry: the alpha-test variants
+    // the tick is of one two-level scene, `scene`, and not in a graph, whose launches keep their
+    // arguments: the OneScene variants
+    bool one_scene;
+    SceneRef scene;
 };
 
 // The path vertices whose shading is sorted when the engine chooses: sorting pays where several
@@ -881,9 +897,9 @@ Grids launch_grids() {
     Grids g;
     g.grid = num_sms() * 8;
     // the alpha variants have the same launch bounds, hence the same residency
-    g.trace = persistent_grid(k_trace<false, false, false>);
-    g.trace2 = persistent_grid(k_trace<false, true, false>);
-    g.trace_c = persistent_grid(k_trace<true, true, false>);
+    g.trace = persistent_grid(k_trace<false, false, false, RayScene>);
+    g.trace2 = persistent_grid(k_trace<false, true, false, RayScene>);
+    g.trace_c = persistent_grid(k_trace<true, true, false, RayScene>);
     g.primary = persistent_grid(k_primary);
     g.shade_p = persistent_grid(k_shade_primary);
     g.shade = persistent_grid(k_shade);
@@ -911,25 +927,40 @@ void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k,
                   unsigned long long* work_ctr, bool sort, cudaStream_t st) {
     const int gr = work_ctr ? g.trace_c : tp.two_level ? g.trace2 : g.trace;
     const int so = sort ? 1 : 0;
-    auto go = [&](auto kernel) { launch(kernel, gr, 128, st, ta, k, qi, parts, work_ctr, so); };
+    auto go = [&](auto kernel, auto scene) {
+        launch(kernel, gr, 128, st, ta, scene, k, qi, parts, work_ctr, so);
+    };
+    const OneScene one{tp.scene};
+    if (tp.one_scene && !work_ctr) {
+        if (tp.alpha) go(k_trace<false, true, true, OneScene>, one);
+        else go(k_trace<false, true, false, OneScene>, one);
+        return;
+    }
     switch ((work_ctr ? 4 : 0) | (tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
-    case 0: go(k_trace<false, false, false>); break;
-    case 1: go(k_trace<false, false, true>); break;
-    case 2: go(k_trace<false, true, false>); break;
-    case 3: go(k_trace<false, true, true>); break;
-    case 4: go(k_trace<true, false, false>); break;
-    case 5: go(k_trace<true, false, true>); break;
-    case 6: go(k_trace<true, true, false>); break;
-    default: go(k_trace<true, true, true>); break;
+    case 0: go(k_trace<false, false, false, RayScene>, RayScene{}); break;
+    case 1: go(k_trace<false, false, true, RayScene>, RayScene{}); break;
+    case 2: go(k_trace<false, true, false, RayScene>, RayScene{}); break;
+    case 3: go(k_trace<false, true, true, RayScene>, RayScene{}); break;
+    case 4: go(k_trace<true, false, false, RayScene>, RayScene{}); break;
+    case 5: go(k_trace<true, false, true, RayScene>, RayScene{}); break;
+    case 6: go(k_trace<true, true, false, RayScene>, RayScene{}); break;
+    default: go(k_trace<true, true, true, RayScene>, RayScene{}); break;
     }
 }
 
 void launch_trace_pixels(const TickArgs& ta, const TickPlan& tp, int grid, cudaStream_t st) {
+    const OneScene one{tp.scene};
+    auto go = [&](auto kernel, auto scene) { launch(kernel, grid, 128, st, ta, scene); };
+    if (tp.one_scene) {
+        if (tp.alpha) go(k_trace_pixels<true, true, OneScene>, one);
+        else go(k_trace_pixels<true, false, OneScene>, one);
+        return;
+    }
     switch ((tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
-    case 0: launch(k_trace_pixels<false, false>, grid, 128, st, ta); break;
-    case 1: launch(k_trace_pixels<false, true>, grid, 128, st, ta); break;
-    case 2: launch(k_trace_pixels<true, false>, grid, 128, st, ta); break;
-    default: launch(k_trace_pixels<true, true>, grid, 128, st, ta); break;
+    case 0: go(k_trace_pixels<false, false, RayScene>, RayScene{}); break;
+    case 1: go(k_trace_pixels<false, true, RayScene>, RayScene{}); break;
+    case 2: go(k_trace_pixels<true, false, RayScene>, RayScene{}); break;
+    default: go(k_trace_pixels<true, true, RayScene>, RayScene{}); break;
     }
 }
 
@@ -1063,7 +1094,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     DevScene* scenes = (DevScene*)(sb + lay.scenes);
     ChunkGPU* chunks = (ChunkGPU*)(sb + lay.chunks);
     e.scene_ptrs.clear();
-    TickPlan tp{0, 0, 0, 1, 1, 0, false, false, false};
+    TickPlan tp{0, 0, 0, 1, 1, 0, false, false, false, false, {}};
     int sort_kinds = 0; // BSDF models in one of the scenes
     bool sort_on = false, sort_auto = false;
     uint64_t paths = 0, pix = 0;
@@ -1114,6 +1145,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     if (tp.n_chunks == 0) return GBPT_OK;
     tp.n_pix = (uint32_t)pix;
     tp.n_paths = (uint32_t)paths;
+    tp.scene = SceneRef{chunks[0].nodes, chunks[0].tris, chunks[0].insts, chunks[0].tri_stride};
     uint32_t sum_lanes = 1;
     while (sum_lanes < std::min(max_spp, 32u)) sum_lanes *= 2;
     tp.sum_lanes = sum_lanes;
@@ -1121,6 +1153,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
 
     // work buffers: a whole wave when graphs replay the tick (their pointers must not move)
     bool graph = e.use_graphs && prof->level == 0;
+    tp.one_scene = tp.two_level && e.scene_ptrs.size() == 1 && !graph;
     if ((rc = work_reserve(w, graph ? wave : paths, graph ? wave : pix)) != GBPT_OK) return rc;
     if (w.perm) tp.sorted = sort_on ? tp.max_len : sort_auto ? sorted_vertices(tp, sort_kinds) : 0u;
     unsigned char* tb = (unsigned char*)w.tables;
@@ -1298,7 +1331,7 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     ta.refill_lanes = (int)sched.refill_lanes;
     ta.postpone_lanes = (int)sched.postpone_lanes;
     const Grids g = launch_grids();
-    TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha};
+    TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha, false, {}};
     cudaMemsetAsync(w.counters + kVertexWord, 0, 4 * sizeof(uint32_t), st);
     launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((P + 127) / 128, (uint64_t)g.trace), st);
     launch(k_primary, (int)((P + 127) / 128), 128, st, ta, 0);
