@@ -943,7 +943,7 @@ static int use_two_streams(gbpt_ctx* ctx, const Profile* prof, bool* two) {
 
 static int render_impl(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam,
                        const gbpt_render_params* p, float* out_dev, float* out_host,
-                       gbpt_render_stats* stats) {
+                       gbpt_render_stats* stats, const gbpt_gbuffer_texel* gbuffer = nullptr) {
     int rc = check_ctx(ctx);
     if (rc) return rc;
     if ((rc = validate_params(cam, p))) return rc;
@@ -961,6 +961,9 @@ static int render_impl(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam,
     a.params.sort_materials = sort_mode(ctx->tuning.sort_materials);
     a.pixel_count = n_pix;
     a.pixels_device = nullptr;
+    // the albedo that "demodulate albedo" divides by needs the unrounded hit
+    if (!p->pixel_count && !p->demodulate_albedo && gbuffer_holds_hits(it->second))
+        a.gbuffer = gbuffer;
     if (p->pixel_count) {
         if (p->pixel_count > w.pix_id_cap) {
             if (w.pix_id) cudaFree(w.pix_id);
@@ -1098,6 +1101,16 @@ GBPT_API int gbpt_render_device(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera
     }
     return render_impl(ctx, scene, camera, params, out_rgba_device, nullptr, stats);
 }
+
+} // extern "C"
+
+int gbpt::render_with_gbuffer(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,
+                              const gbpt_render_params* params, float* out_rgba_device,
+                              const gbpt_gbuffer_texel* gbuffer) {
+    return render_impl(ctx, scene, camera, params, out_rgba_device, nullptr, nullptr, gbuffer);
+}
+
+extern "C" {
 
 // Render through the library's fixed scratch array: no device allocation on this path.
 GBPT_API int gbpt_render_device_noalloc(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,

@@ -81,6 +81,11 @@ int check_ctx(gbpt_ctx* ctx);
 int validate_params(const gbpt_camera* cam, const gbpt_render_params* p);
 // Seconds on the host's steady clock (request timestamps).
 double host_clock();
+// gbpt_render_device whose primary hits are those of `gbuffer` (may be null), the texels that
+// gbpt_gbuffer wrote on the context stream for the same scene, camera, extent and mask.
+int render_with_gbuffer(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,
+                        const gbpt_render_params* params, float* out_rgba_device,
+                        const gbpt_gbuffer_texel* gbuffer);
 // The GBuffer node's emission image: n RGBA32F texels (alpha 1) from n GBuffer texels, device
 // memory, enqueued on the context stream (nodes.cu).
 int gbuffer_emission(gbpt_ctx* ctx, const gbpt_gbuffer_texel* texels, float* out_device,

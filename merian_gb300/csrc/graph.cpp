@@ -59,6 +59,9 @@ struct Buffer {
     uint32_t floats = 4; // floats per texel
     // a scene node's "scene" output: the resident scene and its camera
     bool is_scene = false;
+    // ... and what a GBuffer node's "gbuffer" output was last traced with
+    bool is_gbuffer = false;
+    uint32_t mask = 0;
     uint32_t scene = 0;
     gbpt_camera camera{};
     Buffer() = default;
@@ -333,7 +336,12 @@ class GBufferNode : public Node {
         scene_of(in, scene, camera);
         Buffer& g = out("gbuffer");
         auto* texels = (gbpt_gbuffer_texel*)g.dev;
+        g.is_gbuffer = false;
         check_rc(gbpt_gbuffer(ctx, scene, camera, g.width, g.height, mask(), texels));
+        g.is_gbuffer = true;
+        g.mask = mask();
+        g.scene = scene;
+        g.camera = *camera;
         check_rc(gbuffer_emission(ctx, texels, (float*)out("emission").dev, g.texels()));
     }
 };
@@ -395,7 +403,14 @@ class RenderPTNode : public Node {
         p.frame = (uint32_t)((uint64_t)i("seed") + iteration);
         p.nee = b("next event estimation");
         p.rr_depth = (int32_t)i("russian roulette depth");
-        check_rc(gbpt_render_device(ctx, scene, camera, &p, (float*)o.dev, nullptr));
+        // a G-buffer of the same view holds the primary hits
+        const Buffer* g = input(in, "gbuffer");
+        const bool same_view = g && g->is_gbuffer && g->scene == scene &&
+                               g->mask == p.instance_mask && g->width == o.width &&
+                               g->height == o.height &&
+                               std::memcmp(&g->camera, camera, sizeof(*camera)) == 0;
+        check_rc(render_with_gbuffer(ctx, scene, camera, &p, (float*)o.dev,
+                                     same_view ? (const gbpt_gbuffer_texel*)g->dev : nullptr));
     }
 };
 

@@ -139,6 +139,12 @@ struct Work {
     uint64_t generation = 0;
 };
 
+// Whether a G-buffer texel names any hit of the scene: its geometry and instance indices are 16 bits
+// wide, all ones on a miss.
+inline bool gbuffer_holds_hits(const SceneGPU& s) {
+    return s.geom_count <= 0xFFFFu && s.n_inst <= 0xFFFFu;
+}
+
 // How a request's shading is ordered (BatchItem::params.sort_materials): as the engine finds it
 // faster, or always / never by the tuning. Results do not depend on it.
 constexpr int32_t kSortOff = 0, kSortOn = 1, kSortAuto = 2;
@@ -152,6 +158,9 @@ struct BatchItem {
     const uint32_t* pixels_device = nullptr; // nullptr: all pixels, row-major
     uint32_t pixel_count = 0;
     float4* out_device = nullptr;
+    // the whole image's G-buffer of the same scene, camera, extent and mask (gbuffer_holds_hits):
+    // its hits are the primary hits
+    const gbpt_gbuffer_texel* gbuffer = nullptr;
 };
 
 // Paths per wave: 8 Mi paths keep ~1.5 GB of path state and queues resident.
@@ -179,6 +188,7 @@ struct RenderArgs {
     const uint32_t* pixels_device; // nullptr: all pixels
     uint32_t pixel_count;
     float4* out_device;
+    const gbpt_gbuffer_texel* gbuffer = nullptr; // as BatchItem's
 };
 
 // A request as the tick engine sees it: its pixels are scheduled in list order, whole pixels

@@ -198,6 +198,30 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
 }
 
+// The primary hits of a tick of one request from its G-buffer (BatchItem::gbuffer), whose
+// barycentrics are rounded to half as k_primary rounds them. A pass over 16 of a texel's 64 bytes
+// in place of the traversal (960x540 soup frame: 360 us).
+__global__ void __launch_bounds__(128) k_hits_from_gbuffer(TickArgs t,
+                                                           const gbpt_gbuffer_texel* texels) {
+    wait_for_predecessor();
+    const ChunkGPU& c = t.chunks[0];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < t.hdr->n_pix; q += stride) {
+        // instance and primitive ids, 16-bit geometry and instance indices, half barycentrics
+        const uint2* w = (const uint2*)(texels + c.pix_first + q);
+        const uint2 ids = w[1], hb = w[2];
+        Hit h;
+        const bool ok = ids.x != kNoInst;
+        h.t = 0.0f; // not read
+        h.u = half_lo(hb.y);
+        h.v = half_hi(hb.y);
+        h.prim = ids.y;
+        h.geom = ok ? ids.x + (hb.x & 0xFFFFu) : kNoInst;
+        h.inst = ok && c.insts ? hb.x >> 16 : kNoInst;
+        store_hit(t.w.hit, q, h);
+    }
+}
+
 // The shading point of each pixel slot's primary hit (gbuffer_rt.slang:18-58,
 // render_pt.slang:98-103).
 __global__ void __launch_bounds__(128, kShadeBlocksPerSM) k_primary(TickArgs t, int sort) {
@@ -865,6 +889,7 @@ struct TickPlan {
     // arguments: the OneScene variants
     bool one_scene;
     SceneRef scene;
+    const gbpt_gbuffer_texel* gbuffer; // the one request's, not in a graph
 };
 
 // The path vertices whose shading is sorted when the engine chooses: sorting pays where several
@@ -981,10 +1006,14 @@ uint64_t enqueue_tick(const TickArgs& ta, const TickPlan& tp, const Grids& g, cu
         cudaMemsetAsync(ctr + kSortWord, 0, (tp.sorted + 1) * 8 * sizeof(uint32_t), st);
     const int pgrid = (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.primary);
     int ev = prof->begin(st, 3);
-    launch_trace_pixels(ta, tp,
-                        (int)std::min<uint64_t>((pix + 127) / 128,
-                                                (uint64_t)(tp.two_level ? g.trace2 : g.trace)),
-                        st);
+    if (tp.gbuffer)
+        launch(k_hits_from_gbuffer, (int)std::min<uint64_t>((pix + 127) / 128, (uint64_t)g.grid),
+               128, st, ta, tp.gbuffer);
+    else
+        launch_trace_pixels(ta, tp,
+                            (int)std::min<uint64_t>((pix + 127) / 128,
+                                                    (uint64_t)(tp.two_level ? g.trace2 : g.trace)),
+                            st);
     launch(k_primary, pgrid, 128, st, ta, tp.sorted >= 1 ? 1 : 0);
     prof->end(st, ev);
     nl += 2;
@@ -1094,7 +1123,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     DevScene* scenes = (DevScene*)(sb + lay.scenes);
     ChunkGPU* chunks = (ChunkGPU*)(sb + lay.chunks);
     e.scene_ptrs.clear();
-    TickPlan tp{0, 0, 0, 1, 1, 0, false, false, false, false, {}};
+    TickPlan tp{0, 0, 0, 1, 1, 0, false, false, false, false, {}, nullptr};
     int sort_kinds = 0; // BSDF models in one of the scenes
     bool sort_on = false, sort_auto = false;
     uint64_t paths = 0, pix = 0;
@@ -1154,6 +1183,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     // work buffers: a whole wave when graphs replay the tick (their pointers must not move)
     bool graph = e.use_graphs && prof->level == 0;
     tp.one_scene = tp.two_level && e.scene_ptrs.size() == 1 && !graph;
+    if (n_items == 1 && !graph) tp.gbuffer = items[0]->gbuffer;
     if ((rc = work_reserve(w, graph ? wave : paths, graph ? wave : pix)) != GBPT_OK) return rc;
     if (w.perm) tp.sorted = sort_on ? tp.max_len : sort_auto ? sorted_vertices(tp, sort_kinds) : 0u;
     unsigned char* tb = (unsigned char*)w.tables;
@@ -1268,6 +1298,7 @@ int render_frame(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaStr
     it.pixels_device = args.pixels_device;
     it.pixel_count = args.pixel_count;
     it.out_device = args.out_device;
+    it.gbuffer = args.gbuffer;
     TickEngine e;
     e.work = &w;
     e.stream = st;
@@ -1331,7 +1362,7 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     ta.refill_lanes = (int)sched.refill_lanes;
     ta.postpone_lanes = (int)sched.postpone_lanes;
     const Grids g = launch_grids();
-    TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha, false, {}};
+    TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha, false, {}, nullptr};
     cudaMemsetAsync(w.counters + kVertexWord, 0, 4 * sizeof(uint32_t), st);
     launch_trace_pixels(ta, tp, (int)std::min<uint64_t>((P + 127) / 128, (uint64_t)g.trace), st);
     launch(k_primary, (int)((P + 127) / 128), 128, st, ta, 0);

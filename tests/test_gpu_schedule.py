@@ -222,3 +222,34 @@ def test_rays_with_special_values(gpu_ctx):
                     assert np.array_equal(g[f].view(np.uint32), o[f].view(np.uint32)), f
     finally:
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("kind", ["room", "instanced", "alpha", "alpha-instanced"])
+@pytest.mark.parametrize("case", ["same view", "demodulated", "other mask"])
+def test_primary_hits_from_a_graph_gbuffer(gpu_ctx, kind, case):
+    """A renderer behind a G-buffer node of the same view takes its primary hits from the texels;
+    one whose view or options differ traces them: both equal a render without a G-buffer."""
+    from merian_gb300 import node
+    from merian_gb300 import scene as S
+    sc, (pos, target, fov) = _scenes()[kind]
+    sid = gpu_ctx.upload(sc)
+    try:
+        for w, h, spp in [(33, 3, 1), (129, 67, 2)]:
+            cam = S.look_at(pos, target, (0.0, 1.0, 0.0), fov, w / h)
+            demod = case == "demodulated"
+            props = {"samples per pixel": spp, "max path length": 4, "seed": 5,
+                     "demodulate albedo": demod, "next event estimation": True}
+            gp = {"width": w, "height": h}
+            if case == "other mask":
+                gp.update({str(b): False for b in range(8)})
+            with node.Graph(gpu_ctx, {"nodes": {
+                    "g": {"type": "GBuffer (Raytraced)", "properties": gp,
+                          "outputs": ["gbuffer->r.gbuffer"]},
+                    "r": {"type": "Render (Path-traced)", "properties": props}}}) as g:
+                g.run(sid, cam, (w, h), 2)
+                out = g.output("r.irradiance").reshape(-1, 4)
+            p, _ = S.render_params(w, h, spp, 4, nee=True, frame=6, demodulate_albedo=demod)
+            ref = gpu_ctx.render(sid, cam, p)
+            assert np.array_equal(out.view(np.uint32), ref.view(np.uint32)), (w, h)
+    finally:
+        gpu_ctx.destroy_scene(sid)
