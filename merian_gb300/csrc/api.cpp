@@ -17,6 +17,9 @@
 #include <string>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cuda_runtime.h>
 
 namespace gbpt {
@@ -884,6 +887,17 @@ GBPT_API int gbpt_scene_stats(gbpt_ctx* ctx, uint32_t scene, uint64_t* nodes, ui
 
 } // extern "C"
 
+void gbpt::prefault_host(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+    if (bytes < (256u << 10)) return; // a few pages fault faster than they are asked for
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(page - 1);
+    madvise((void*)a, (uintptr_t)p + bytes - a, MADV_POPULATE_WRITE);
+#else
+    (void)p;
+    (void)bytes;
+#endif
+}
+
 int gbpt::validate_params(const gbpt_camera* cam, const gbpt_render_params* p) {
     if (!cam || !p) {
         set_error("null camera or params");
@@ -1023,6 +1037,7 @@ static int render_impl(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam,
     }
     if (stats) GBPT_CUDA_CHECK(cudaEventRecord(ctx->ev1, ctx->stream));
     if (out_host) {
+        prefault_host(out_host, (size_t)n_pix * sizeof(float4));
         GBPT_CUDA_CHECK(cudaMemcpyAsync(out_host, a.out_device, (size_t)n_pix * sizeof(float4),
                                         cudaMemcpyDeviceToHost, ctx->stream));
     }
@@ -1252,6 +1267,9 @@ GBPT_API int gbpt_render_batch(gbpt_ctx* ctx, const gbpt_request* reqs, uint32_t
         return rc;
     }
     if (stats) GBPT_CUDA_CHECK(cudaEventRecord(ctx->ev1, ctx->stream));
+    for (uint32_t i = 0; i < n; ++i)
+        if (reqs[i].out_host)
+            prefault_host(reqs[i].out_host, (size_t)items[i].pixel_count * sizeof(float4));
     for (uint32_t i = 0; i < n; ++i) {
         if (!reqs[i].out_host) continue;
         GBPT_CUDA_CHECK(cudaMemcpyAsync(reqs[i].out_host, items[i].out_device,
@@ -1560,6 +1578,7 @@ GBPT_API int gbpt_trace_primary(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera
         set_error("gbpt_trace_primary: launch failed");
         return rc;
     }
+    prefault_host(out_hits_host, n * sizeof(gbpt_hit));
     GBPT_CUDA_CHECK(cudaMemcpyAsync(out_hits_host, ctx->d_hits, n * sizeof(gbpt_hit),
                                     cudaMemcpyDeviceToHost, ctx->stream));
     return check_device_error(ctx);

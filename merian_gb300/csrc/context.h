@@ -81,6 +81,11 @@ int check_ctx(gbpt_ctx* ctx);
 int validate_params(const gbpt_camera* cam, const gbpt_render_params* p);
 // Seconds on the host's steady clock (request timestamps).
 double host_clock();
+// Makes the pages of a host output present while the GPU is still rendering into its device side:
+// a copy to fresh memory otherwise takes a page fault per page in the copy (67 MB of new pages:
+// 3.8 ms, present ones 0.4). Leaves contents as they are; memory that cannot be populated
+// is left to the copy.
+void prefault_host(void* p, size_t bytes);
 // gbpt_render_device whose primary hits are those of `gbuffer` (may be null), the texels that
 // gbpt_gbuffer wrote on the context stream for the same scene, camera, extent and mask.
 int render_with_gbuffer(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,

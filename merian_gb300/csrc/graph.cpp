@@ -1441,6 +1441,7 @@ GBPT_API int gbpt_graph_output(gbpt_graph* graph, const char* connector, float* 
         std::copy(b->host.begin(), b->host.begin() + (ptrdiff_t)count, out_host);
         return GBPT_OK;
     }
+    prefault_host(out_host, count * sizeof(float));
     int rc = gbpt_synchronize(graph->ctx);
     if (rc) return rc;
     GBPT_CUDA_CHECK(cudaMemcpy(out_host, b->dev, count * sizeof(float), cudaMemcpyDeviceToHost));
