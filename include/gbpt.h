@@ -341,10 +341,8 @@ typedef struct gbpt_tuning {
     /* warp scheduling of the persistent traversal launches, 0 = default each */
     int32_t trace_refill_lanes;   /* a warp refills its idle lanes with new rays once fewer than
                                      this many lanes are busy: [1, 32], default 20 */
-    int32_t trace_postpone_lanes; /* a lane pushes its triangle group for later when fewer than
-                                     this many lanes have triangles to test: [1, 32], default 6;
-                                     closest-hit traversal only (a first-hit query tests its
-                                     triangles at once) */
+    int32_t trace_postpone_lanes; /* [1, 32], default 6: kept for its callers, without effect (the
+                                     traversal tests its triangles at once) */
     int32_t trace_blocks_per_sm;  /* 128-thread blocks per SM of the traversal launches: [1, 64],
                                      capped at what is resident; default all resident */
 } gbpt_tuning;
@@ -528,8 +526,7 @@ GBPT_API int gbpt_graph_output(gbpt_graph* graph, const char* connector, float* 
  * (gbuffer_rt.slang:18-58) with full-precision barycentrics and t, written to a host array of
  * width*height records. gbpt_trace: closest-hit (any_hit = 0) or occlusion (any_hit = 1, only
  * t is written: 0 = occluded, -1 = clear) for n device-resident rays, on the context tuning's
- * traversal schedule (trace_* fields; with trace_postpone_lanes = 1 no triangle group is
- * postponed, so nodes and triangles are visited in the order of a one-ray-at-a-time walk). */
+ * traversal schedule (trace_* fields). */
 GBPT_API int gbpt_trace_primary(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,
                                 uint32_t width, uint32_t height, uint32_t instance_mask,
                                 gbpt_hit* out_hits_host);

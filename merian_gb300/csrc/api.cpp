@@ -76,7 +76,6 @@ cudaError_t device_malloc(void** p, size_t bytes) {
 TraceSched sched_of(const gbpt_tuning& t) {
     TraceSched s;
     if (t.trace_refill_lanes > 0) s.refill_lanes = (uint32_t)t.trace_refill_lanes;
-    if (t.trace_postpone_lanes > 0) s.postpone_lanes = (uint32_t)t.trace_postpone_lanes;
     if (t.trace_blocks_per_sm > 0) s.blocks_per_sm = (uint32_t)t.trace_blocks_per_sm;
     return s;
 }
@@ -427,8 +426,7 @@ static int build_scene_bvh(const gbpt_scene_desc* d, int32_t bvh_build, CwBvh& b
         bi.geom.reserve(total_tris);
         bi.flags.reserve(total_tris);
         if ((rc = gather(0, d->geometry_count, bi))) return rc;
-        // each tree level puts at most one node group and one postponed triangle group on the
-        // 48-entry traversal stack
+        // each tree level puts at most one node group on the 48-entry traversal stack
         if (!build_cwbvh(bi, bvh, 24)) return GBPT_ERR_INVALID;
     } else {
         // one CWBVH per BLAS in object space, a top-level CWBVH over the instances' world boxes
@@ -1340,7 +1338,8 @@ GBPT_API int gbpt_get_tuning(gbpt_ctx* ctx, gbpt_tuning* t) {
 // The autotuner: candidate tunings rendered on one representative request, the fastest kept.
 // Outputs do not depend on the tuning (tick size, shading order and warp scheduling only change
 // the schedule), so only time is compared. Stage 1 crosses tick size and material sorting; the
-// traversal's refill and postponement thresholds and its blocks per SM are then searched one at a
+// traversal's refill threshold, the postponement threshold (now without effect: its candidates tie)
+// and its blocks per SM are then searched one at a
 // time from the best so far. Results are cached per bucket of scene size, frame size, path length
 // and estimator.
 GBPT_API int gbpt_autotune(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,
@@ -1432,7 +1431,7 @@ GBPT_API int gbpt_autotune(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam
     {
         const TraceSched defaults;
         best.trace_refill_lanes = (int32_t)defaults.refill_lanes;
-        best.trace_postpone_lanes = (int32_t)defaults.postpone_lanes;
+        best.trace_postpone_lanes = 6; // without effect
         best.trace_blocks_per_sm = 0; // every resident block
     }
     double best_ms = 1e300;

@@ -247,7 +247,7 @@ GBPT_DI bool intersect_tri(const RayPre& p, float4 a4, float4 b4, float4 c4, uin
 
 // ---- CWBVH traversal ----------------------------------------------------------------------------
 // Traversal stack entries per ray. The builder bounds the tree depth (24 levels), which with
-// postponed triangle groups and instance entries stays below the default. A build with a smaller
+// instance entries stays below the default. A build with a smaller
 // GBPT_STACK_SIZE makes deep traversals overflow: the overflow sets the kernels' error word
 // (GBPT_ERR_DEVICE on the host) and finishes the ray with what it found, never a fault, so the
 // error path can be exercised on purpose.
@@ -294,15 +294,17 @@ GBPT_DI float3 xform_vector(float4 r0, float4 r1, float4 r2, float3 v) {
 }
 
 // ---- traversal state and loop ------------------------------------------------------------------
-// One loop serves every query (trace_persistent): a lane postpones its pending triangle tests
-// (pushes the triangle group onto its stack) when fewer than `postpone_lanes` lanes of the warp
-// have triangles to test, so node steps and triangle steps stay in lockstep across the warp, and
-// the warp leaves the loop to refill idle lanes once fewer than `refill_lanes` lanes are busy
-// (both launch arguments). Two-level scenes: a top-level leaf is an instance; entering it pushes
-// what is left of the top level, transforms the ray to object space (t is unchanged: the
-// direction is not renormalised) and continues from the BLAS root; when the stack drops back to
-// the entry depth the world ray is restored. The closest hit and the tie rule (equal t: smallest
-// geometry, primitive, instance) do not depend on the visit order.
+// One loop serves every query (trace_persistent): a node step, the triangles of the leaves it hit,
+// then the next group off the stack; the warp leaves it to refill idle lanes once fewer than
+// `refill_lanes` lanes are busy (a launch argument). Two-level scenes: a top-level leaf is an
+// instance; entering it pushes what is left of the top level, transforms the ray to object space
+// (t is unchanged: the direction is not renormalised) and continues from the BLAS root; when the
+// stack drops back to the entry depth the world ray is restored. The closest hit and the tie rule
+// (equal t: smallest geometry, primitive, instance) do not depend on the visit order.
+// The loop is kept short: postponing triangle groups until several lanes of a warp had some to
+// test, and sharing rays only every other step, each cost more instructions a step than they
+// saved (1080p soup frame 251.9 ms with both, 244.7 without the first, 240.4 without either; a
+// million closest hits 0.82 / 0.75 / 0.72 ms).
 
 
 struct TraceState {
@@ -321,7 +323,7 @@ struct TraceState {
     uint32_t inst; // instance being traversed, kNoInst at the top level
     int inst_sp;   // stack depth at which it was entered
     // bits 0-7: the stack's first entry of this lane (those below were given to other lanes);
-    // bits 8-12: the lane that keeps the ray's result; bits 16 up: steps of the current run
+    // bits 8-12: the lane that keeps the ray's result
     uint32_t aux;
     GBPT_DI int floor() const { return (int)(aux & 0xFFu); }
     GBPT_DI uint32_t owner() const { return (aux >> 8) & 31u; }
@@ -376,10 +378,12 @@ GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tma
     set_ray(s, o, d);
     s.wo = o;
     s.wd = d;
-    s.tmin = tmin;
-    // a span with a NaN end holds no hit (and would make every box test a hit)
-    s.ngroup = make_uint2(0u, tmin == tmin && tmax == tmax ? 0x80000000u : 0u);
+    // a span with a NaN end holds no hit, but would make every box test one: an empty span
+    const bool span = tmin == tmin && tmax == tmax;
+    if (!span) tmin = 0.0f, tmax = -1.0f;
+    s.ngroup = make_uint2(0u, 0x80000000u);
     s.tgroup = make_uint2(0u, 0u);
+    s.tmin = tmin;
     s.best.t = tmax;
     s.best.u = s.best.v = 0.0f;
     s.best.prim = s.best.geom = s.best.inst = kNoInst;
@@ -582,22 +586,17 @@ GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni
 template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class Scene, class StackRef, class Alpha>
 GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const OctantOrder& order,
                         TraceCounters* ctr, uint32_t* err,
-                        const Alpha& alpha, int min_lanes, uint32_t step_mask,
-                        int postpone_lanes) {
+                        const Alpha& alpha, int min_lanes) {
     while (true) {
-        const bool any = MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u);
-        if (s.ngroup.y > 0x00FFFFFFu) {
+        // without instances the stack holds node groups only
+        if (!TWO_LEVEL || s.ngroup.y > 0x00FFFFFFu) {
             const uint32_t hits = s.ngroup.y;
             const uint32_t bit = 31u - __clz(hits & 0xFF000000u);
             s.ngroup.y &= ~(1u << bit);
             if (s.ngroup.y > 0x00FFFFFFu) {
                 if (s.sp() >= kStackSize) {
                     atomicOr(err, 1u);
-                    s.clear_sp();
-                    s.ngroup.y = 0;
-                    s.tgroup.y = 0;
-                    s.inst = kNoInst;
-                    break;
+                    return true;
                 }
                 st(s.sp()) = s.ngroup;
                 s.push_sp();
@@ -610,22 +609,11 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(
                 s, scene.nodes(s), ni, order, s.ngroup, s.tgroup, ctr);
         } else {
-            // a postponed triangle group (or the rest of a top-level instance group) came off
-            // the stack
+            // the rest of a top-level instance group came off the stack
             s.tgroup = s.ngroup;
             s.ngroup = make_uint2(0u, 0u);
         }
-        bool done_any = false;
-        // only groups followed by node work are postponed (a group popped back is tested), and
-        // never those of a first-hit query, which any of its triangles may end
-        const bool may_postpone = !any && s.ngroup.y > 0x00FFFFFFu;
         while (s.tgroup.y != 0u) {
-            if (may_postpone && s.sp() < kStackSize && __popc(__activemask()) < postpone_lanes) {
-                st(s.sp()) = s.tgroup;
-                s.push_sp();
-                s.tgroup.y = 0u;
-                break;
-            }
             const uint32_t b = __ffs(s.tgroup.y) - 1u;
             s.tgroup.y &= s.tgroup.y - 1u;
             const uint32_t ti = s.tgroup.x + b;
@@ -681,27 +669,19 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
                 s.best.geom = geom;
                 s.best.inst = s.inst;
                 if (MODE != kTraceAny) s.pre.k = (s.pre.k & ~kTriKey) | (tfl & kTriKey);
-                if (any) {
-                    done_any = true;
-                    break;
-                }
+                // a first-hit ray ends with it
+                if (MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u))
+                    return true;
             }
         }
-        bool done = done_any;
-        if (!done && s.ngroup.y <= 0x00FFFFFFu) {
+        if (s.ngroup.y <= 0x00FFFFFFu) {
             if (TWO_LEVEL && s.inst != kNoInst && s.sp() == s.inst_sp) exit_instance(s);
-            if (s.sp() == s.floor()) {
-                done = true;
-            } else {
-                s.pop_sp();
-                s.ngroup = st(s.sp());
-            }
+            if (s.sp() == s.floor()) return true;
+            s.pop_sp();
+            s.ngroup = st(s.sp());
         }
-        if (done) break;
-        s.aux += 1u << 16;
-        if ((s.aux & step_mask) == 0u && __popc(__activemask()) < min_lanes) return false;
+        if (__popc(__activemask()) < min_lanes) return false;
     }
-    return true;
 }
 
 // Position of the r-th set bit of m (r < popc(m)).
@@ -741,10 +721,6 @@ GBPT_DI bool hit_before(float t, uint32_t geom, uint32_t prim, uint32_t inst, co
 // frame of path length 16 takes 5.56 / 4.41 ms, 37,003 pixels x 8 of the 200k-triangle soup 2.17 /
 // 1.79, a 64x64 frame of the room 0.30 / 0.25; where queues are long it is neutral (1080p soup
 // frame 261.5 / 260.6).
-// Steps between two shares: 1 / 2 / 4 / 8 measure 4.31 / 4.41 / 4.53 / 4.74 ms on the instanced
-// frame, 1.81 / 1.79 / 1.79 / 1.86 on the pixel list, 260.6 / 260.8 / 261.5 (2 / 4 / 8) on the 1080p
-// soup.
-constexpr uint32_t kShareSteps = 2; // a power of two
 template <TraceMode MODE, bool TWO_LEVEL, bool PER_RAY, class StackRef, class Store>
 GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& active, bool& owns,
                         const Store& store) {
@@ -862,8 +838,7 @@ template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, bool SHARE, class Scene, c
 __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n, uint32_t* fetch,
                                                  Load load,
                                                  Store store_hit, Alpha alpha, TraceCounters* ctr,
-                                                 uint32_t* err, int refill_lanes,
-                                                 int postpone_lanes) {
+                                                 uint32_t* err, int refill_lanes) {
     const uint32_t lane = threadIdx.x & 31u;
     __shared__ OctantOrder order;
     octant_order_init(order);
@@ -927,13 +902,11 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
         const auto ray_alpha = [&](uint32_t g, uint32_t p, float u, float v) {
             return alpha(ray, g, p, u, v);
         };
-        // until few lanes are busy and the pool can refill the others; with the pool empty a few
-        // steps between two shares, or to the end
-        s.aux &= 0xFFFFu;
+        // until few lanes are busy and the pool can refill the others; with the pool empty a step
+        // between two shares, or to the end
         if (trace_loop<MODE, COUNT, TWO_LEVEL>(
-                s, scene, st_ref, order, ctr, err, ray_alpha, pool_empty ? (SHARE ? 33 : 0) : refill_lanes,
-                SHARE && pool_empty ? (kShareSteps - 1u) << 16 : 0u,
-                postpone_lanes)) {
+                s, scene, st_ref, order, ctr, err, ray_alpha,
+                pool_empty ? (SHARE ? 33 : 0) : refill_lanes)) {
             active = false;
             if (!SHARE || !pool_empty) {
                 store(ray, s);

@@ -45,8 +45,7 @@ GBPT_DI OneScene one_scene(const DevScene& sc) {
 template <bool ANY, bool COUNT, bool TWO_LEVEL, bool ALPHA>
 __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     k_trace_rays(DevScene sc, const gbpt_ray* rays, uint32_t n, uint32_t mask, gbpt_hit* hits,
-                 unsigned long long* work_ctr, uint32_t* fetch, uint32_t* err, int refill_lanes,
-                 int postpone_lanes) {
+                 unsigned long long* work_ctr, uint32_t* fetch, uint32_t* err, int refill_lanes) {
     TraceCounters ctr{0, 0, 0, 0, 0, 0};
     auto load = [&](uint32_t i, TraceState& s) {
         const gbpt_ray r = rays[i];
@@ -60,7 +59,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
     trace_persistent<ANY ? kTraceAny : kTraceClosest, COUNT, TWO_LEVEL, !ANY && !COUNT>(
-        one_scene(sc), n, fetch, load, store, alpha, &ctr, err, refill_lanes, postpone_lanes);
+        one_scene(sc), n, fetch, load, store, alpha, &ctr, err, refill_lanes);
     if (COUNT) {
         atomicAdd(work_ctr + 0, (unsigned long long)ctr.nodes);
         atomicAdd(work_ctr + 1, (unsigned long long)ctr.tris);
@@ -76,8 +75,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
 template <bool TWO_LEVEL, bool ALPHA>
 __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     k_trace_primary(DevScene sc, CamGPU cam, uint32_t w, uint32_t h, uint32_t mask, gbpt_hit* hits,
-                    gbpt_gbuffer_texel* texels, uint32_t* fetch, uint32_t* err, int refill_lanes,
-                    int postpone_lanes) {
+                    gbpt_gbuffer_texel* texels, uint32_t* fetch, uint32_t* err, int refill_lanes) {
     auto load = [&](uint32_t i, TraceState& s) {
         float3 o, d;
         float tmin, tmax;
@@ -103,8 +101,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
     trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(
-        one_scene(sc), w * h, fetch, load, store, alpha, nullptr, err, refill_lanes,
-        postpone_lanes);
+        one_scene(sc), w * h, fetch, load, store, alpha, nullptr, err, refill_lanes);
 }
 
 GBPT_DI uint32_t pack_half2_rn(float lo, float hi) {
@@ -204,7 +201,7 @@ int trace_rays(const SceneGPU& scene, const gbpt_ray* rays, uint32_t n, uint32_t
         int grid = persistent_grid(kernel);
         if (sched.blocks_per_sm) grid = std::min(grid, (int)sched.blocks_per_sm * num_sms());
         kernel<<<grid, 128, 0, st>>>(sc, rays, n, mask & 0xFFu, hits, work_ctr, fetch, err,
-                                     (int)sched.refill_lanes, (int)sched.postpone_lanes);
+                                     (int)sched.refill_lanes);
     };
     if (count) {
         if (any_hit) go(k_trace_rays<true, true, true, true>);
@@ -234,7 +231,7 @@ void launch_trace_primary(const SceneGPU& scene, const DevScene& sc, const CamGP
         int grid = std::min(persistent_grid(kernel), (int)(((uint64_t)w * h + 127) / 128));
         if (sched.blocks_per_sm) grid = std::min(grid, (int)sched.blocks_per_sm * num_sms());
         kernel<<<grid, 128, 0, st>>>(sc, cam, w, h, mask & 0xFFu, hits, texels, fetch, err,
-                                     (int)sched.refill_lanes, (int)sched.postpone_lanes);
+                                     (int)sched.refill_lanes);
     };
     switch ((sc.n_inst ? 2 : 0) | (scene.alpha ? 1 : 0)) {
     case 0: go(k_trace_primary<false, false>); break;

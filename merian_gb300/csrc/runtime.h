@@ -199,13 +199,10 @@ struct TickItem : BatchItem {
 
 // Warp scheduling of the persistent traversal kernels, chosen at launch (gbpt_tuning, searched
 // by the autotuner; results never depend on it): a warp leaves its traversal loop to refill its
-// idle lanes with new rays once fewer than refill_lanes lanes are busy; a lane pushes its
-// triangle group for later when fewer than postpone_lanes lanes of the warp have triangles to
-// test; the closest-hit and any-hit launches run blocks_per_sm blocks of 128 threads per SM
-// (0: every block that is resident at once).
+// idle lanes with new rays once fewer than refill_lanes lanes are busy; the traversal launches run
+// blocks_per_sm blocks of 128 threads per SM (0: every block that is resident at once).
 struct TraceSched {
     uint32_t refill_lanes = 20;
-    uint32_t postpone_lanes = 6;
     uint32_t blocks_per_sm = 0;
 };
 

@@ -93,7 +93,7 @@ struct TickArgs {
     const ChunkGPU* chunks;
     const TickHeader* hdr;
     Work w;
-    int refill_lanes, postpone_lanes; // warp scheduling of the persistent traversal
+    int refill_lanes; // warp scheduling of the persistent traversal
 };
 
 // last chunk whose base <= key
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     };
     trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(
         scene, n, vertex_words(t, 0) + kCursor, load, store, alpha, nullptr, t.w.counters + 3,
-        t.refill_lanes, t.postpone_lanes);
+        t.refill_lanes);
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(t.w.stats + 0, (unsigned long long)n);
 }
 
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
     };
     trace_persistent<kTraceMixed, COUNT, TWO_LEVEL, !COUNT>(
         scene, n_rays + n_shadows, words + (parts == 2 ? kCursor2 : kCursor), load, store, alpha, &ctr,
-        t.w.counters + 3, t.refill_lanes, t.postpone_lanes);
+        t.w.counters + 3, t.refill_lanes);
     if (sort) {
         __syncthreads();
         if (threadIdx.x < kSortKeys && key_count[threadIdx.x])
@@ -1197,7 +1197,6 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     ta.chunks = (const ChunkGPU*)(tb + lay.chunks);
     ta.w = w;
     ta.refill_lanes = (int)e.sched.refill_lanes;
-    ta.postpone_lanes = (int)e.sched.postpone_lanes;
     if (e.grids[0] == 0) {
         const Grids g = launch_grids();
         static_assert(sizeof(Grids) == sizeof(e.grids), "grid cache");
@@ -1360,7 +1359,6 @@ int primary_points(const SceneGPU& scene, Work& w, const RenderArgs& args, cudaS
     ta.w = w;
     const TraceSched sched;
     ta.refill_lanes = (int)sched.refill_lanes;
-    ta.postpone_lanes = (int)sched.postpone_lanes;
     const Grids g = launch_grids();
     TickPlan tp{1, P, P, 1, 1, 0, false, s.n_inst != 0u, scene.alpha, false, {}, nullptr};
     cudaMemsetAsync(w.counters + kVertexWord, 0, 4 * sizeof(uint32_t), st);
