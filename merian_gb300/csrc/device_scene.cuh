@@ -591,8 +591,8 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
         // without instances the stack holds node groups only
         if (!TWO_LEVEL || s.ngroup.y > 0x00FFFFFFu) {
             const uint32_t hits = s.ngroup.y;
-            const uint32_t bit = 31u - __clz(hits & 0xFF000000u);
-            s.ngroup.y &= ~(1u << bit);
+            const uint32_t bit = 31u - __clz(hits);
+            s.ngroup.y = hits ^ (1u << bit);
             if (s.ngroup.y > 0x00FFFFFFu) {
                 if (s.sp() >= kStackSize) {
                     atomicOr(err, 1u);
@@ -602,7 +602,7 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
                 s.push_sp();
             }
             const uint32_t slot = (bit - 24u) ^ s.pre.oct_inv();
-            const uint32_t ni = s.ngroup.x + __popc((hits & 0xFFu) & ((1u << slot) - 1u));
+            const uint32_t ni = s.ngroup.x + __popc(hits & ((1u << slot) - 1u));
             if (COUNT) count_step(ctr->node_steps, ctr->node_lanes);
             // the paired planes hold more registers: first-hit traversal, which keeps fewer,
             // measured faster with the scalar ones

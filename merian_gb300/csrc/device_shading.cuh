@@ -427,9 +427,12 @@ template <class K> int persistent_grid(K kernel) {
 constexpr int kTraceBlocksPerSM = GBPT_TRACE_BLOCKS_PER_SM;
 // The two-level variants keep the world ray and the instance as well: 7 blocks (72 registers) spill
 // less than 8 and beat them (instanced 1280x720 frame, 8 / 7 / 6 / 5 blocks: 4.36 / 4.25 / 4.30 /
-// 4.35 ms); the others are faster with 8 (1080p soup frame, 8 / 7 blocks: 260.8 / 266.9 ms).
-constexpr int trace_blocks(bool two_level) {
-    return two_level ? kTraceBlocksPerSM - 1 : kTraceBlocksPerSM;
+// 4.35 ms). The others run 8, and 9 in long queues, where the ninth block hides more of the others'
+// waiting than its spills cost (1080p soup frame 235.0 instead of 239.8 ms, 640x360 7.65 instead of
+// 7.80); short queues end with a few rays whose latency the spills add to (37,003 pixels x 8 1.68
+// instead of 1.64).
+constexpr int trace_blocks(bool two_level, bool long_queue = false) {
+    return two_level ? kTraceBlocksPerSM - 1 : kTraceBlocksPerSM + (long_queue ? 1 : 0);
 }
 
 } // namespace gbpt

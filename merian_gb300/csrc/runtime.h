@@ -226,7 +226,7 @@ struct TickEngine {
     uint64_t graph_generation = 0; // Work::generation the graphs were captured with
     std::vector<unsigned char> stage;
     std::vector<const SceneGPU*> scene_ptrs;
-    int grids[7] = {0, 0, 0, 0, 0, 0, 0}; // launch grids, computed at the first tick
+    int grids[8] = {0, 0, 0, 0, 0, 0, 0, 0}; // launch grids, computed at the first tick
     void release(); // destroys the graphs
 };
 

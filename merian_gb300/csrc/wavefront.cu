@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
 // 0.28 instead of 0.41 ms, the instanced 1280x720 frame of path length 16 5.6 instead of 7.6, the
 // 640x360 soup frame 8.6 instead of 9.4; the clears of the counters, now one per tick instead of
 // four per vertex, included).
-template <bool COUNT, bool TWO_LEVEL, bool ALPHA, class Scene>
-__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
+template <bool COUNT, bool TWO_LEVEL, bool ALPHA, class Scene, bool LONG = false>
+__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL, LONG))
     k_trace(TickArgs t, Scene scene, int k, int qi, int parts, unsigned long long* work_ctr,
             int sort) {
     wait_for_predecessor();
@@ -912,6 +912,7 @@ uint32_t sorted_vertices(const TickPlan& tp, int kinds) {
 struct Grids {
     int grid;    // grid-stride kernels without a register budget (finalize, material sort)
     int trace;   // persistent traversal: the blocks resident at once
+    int trace_l; // ... of the long-queue variants
     int trace2;  // ... of the two-level variants
     int trace_c; // ... of the counting ones
     int primary; // k_primary, k_shade_primary, k_shade: their resident blocks
@@ -923,6 +924,7 @@ Grids launch_grids() {
     g.grid = num_sms() * 8;
     // the alpha variants have the same launch bounds, hence the same residency
     g.trace = persistent_grid(k_trace<false, false, false, RayScene>);
+    g.trace_l = persistent_grid(k_trace<false, false, false, RayScene, true>);
     g.trace2 = persistent_grid(k_trace<false, true, false, RayScene>);
     g.trace_c = persistent_grid(k_trace<true, true, false, RayScene>);
     g.primary = persistent_grid(k_primary);
@@ -933,6 +935,11 @@ Grids launch_grids() {
 
 // The traversal variants of a tick: work counters, two-level scenes, alpha-tested geometry (the
 // variants without a feature leave its code out; they find the same hits on scenes without it).
+// Ticks of at least this many paths trace with 9 blocks per SM (trace_blocks): between the 0.3 M
+// paths that lose by it and the 3.7 M that gain; at 1 M (256x256 room, 16 samples) both take
+// 1.02 ms.
+constexpr uint32_t kLongTick = 1u << 20;
+
 // A kernel that begins with wait_for_predecessor().
 template <class... P, class... A>
 void launch(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... args) {
@@ -950,7 +957,8 @@ void launch(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... arg
 
 void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k, int qi, int parts,
                   unsigned long long* work_ctr, bool sort, cudaStream_t st) {
-    const int gr = work_ctr ? g.trace_c : tp.two_level ? g.trace2 : g.trace;
+    const bool lng = !work_ctr && !tp.two_level && tp.n_paths >= kLongTick;
+    const int gr = work_ctr ? g.trace_c : tp.two_level ? g.trace2 : lng ? g.trace_l : g.trace;
     const int so = sort ? 1 : 0;
     auto go = [&](auto kernel, auto scene) {
         launch(kernel, gr, 128, st, ta, scene, k, qi, parts, work_ctr, so);
@@ -959,6 +967,11 @@ void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k,
     if (tp.one_scene && !work_ctr) {
         if (tp.alpha) go(k_trace<false, true, true, OneScene>, one);
         else go(k_trace<false, true, false, OneScene>, one);
+        return;
+    }
+    if (lng) {
+        if (tp.alpha) go(k_trace<false, false, true, RayScene, true>, RayScene{});
+        else go(k_trace<false, false, false, RayScene, true>, RayScene{});
         return;
     }
     switch ((work_ctr ? 4 : 0) | (tp.two_level ? 2 : 0) | (tp.alpha ? 1 : 0)) {
@@ -1207,6 +1220,7 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
     if (e.sched.blocks_per_sm > 0) {
         const int cap = (int)e.sched.blocks_per_sm * num_sms();
         grids.trace = std::min(grids.trace, cap);
+        grids.trace_l = std::min(grids.trace_l, cap);
         grids.trace2 = std::min(grids.trace2, cap);
         grids.trace_c = std::min(grids.trace_c, cap);
     }
@@ -1217,7 +1231,8 @@ int tick_enqueue(TickEngine& e, TickItem* const* items, uint32_t n_items, uint64
             e.graph_generation = w.generation;
         }
         const uint32_t shape = (tp.max_len << 16) + (tp.sorted << 8) + (tp.nee ? 1u : 0u) +
-                               (tp.two_level ? 2u : 0u) + (tp.alpha ? 4u : 0u);
+                               (tp.two_level ? 2u : 0u) + (tp.alpha ? 4u : 0u) +
+                               (tp.n_paths >= kLongTick ? 8u : 0u);
         const TickEngine::Graph* found = nullptr;
         for (const auto& g : e.graphs)
             if (g.shape == shape) found = &g;

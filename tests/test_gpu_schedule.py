@@ -253,3 +253,23 @@ def test_primary_hits_from_a_graph_gbuffer(gpu_ctx, kind, case):
             assert np.array_equal(out.view(np.uint32), ref.view(np.uint32)), (w, h)
     finally:
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("kind", ["room", "alpha"])
+@pytest.mark.parametrize("height", [1023, 1024])
+def test_long_and_short_ticks(gpu_ctx, kind, height):
+    """Ticks from 2^20 paths on trace with another register budget: the bits of the same frame in
+    shorter ticks."""
+    from merian_gb300 import scene as S
+    sc, (pos, target, fov) = _scenes()[kind]
+    sid = gpu_ctx.upload(sc)
+    cam = S.look_at(pos, target, (0.0, 1.0, 0.0), fov, 1.0)
+    try:
+        p, _ = S.render_params(1024, height, 1, 4, nee=True, frame=2)
+        a = gpu_ctx.render(sid, cam, p)
+        gpu_ctx.set_tuning(wave_paths=1 << 19)
+        b = gpu_ctx.render(sid, cam, p)
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    finally:
+        gpu_ctx.set_tuning()
+        gpu_ctx.destroy_scene(sid)
