@@ -322,10 +322,11 @@ struct TraceState {
     float3 wo, wd; // the world ray
     uint32_t inst; // instance being traversed, kNoInst at the top level
     int inst_sp;   // stack depth at which it was entered
-    // bits 0-7: the stack's first entry of this lane (those below were given to other lanes);
-    // bits 8-12: the lane that keeps the ray's result
+    // bits 24-31: the stack's first entry of this lane (those below were given to other lanes), as
+    // the depth in the axis word; bits 8-12: the lane that keeps the ray's result
     uint32_t aux;
-    GBPT_DI int floor() const { return (int)(aux & 0xFFu); }
+    GBPT_DI int floor() const { return (int)(aux >> 24); }
+    GBPT_DI bool at_floor() const { return (pre.k ^ aux) < (1u << 24); }
     GBPT_DI uint32_t owner() const { return (aux >> 8) & 31u; }
     // the traversal stack's depth, kept in bits 24..31 of the ray's axis word
     GBPT_DI int sp() const { return (int)(pre.k >> 24); }
@@ -643,14 +644,19 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             const float4 r1 = __ldg(rec + 1);
             const float4 r2 = __ldg(rec + 2);
             const uint32_t tfl = __float_as_uint(r2.w);
-            if ((tfl & s.pre.mask()) == 0u) continue;
             if (COUNT) {
+                if ((tfl & s.pre.mask()) == 0u) continue;
                 ctr->tris++;
                 count_step(ctr->tri_steps, ctr->tri_lanes);
             }
             float t, u, v;
             float det;
             if (!intersect_tri(s.pre, r0, r1, r2, tfl, s.tmin, s.best.t, t, u, v, det)) continue;
+            // the instance mask is tested where few candidates get: before the intersection, it made
+            // every triangle step wait for the flag word and branch once more (1080p soup frame
+            // 235.1 instead of 227.7 ms, a million closest hits 0.72 instead of 0.65). What is
+            // counted is still what passes the mask.
+            if (!COUNT && (tfl & s.pre.mask()) == 0u) continue;
             const uint32_t prim = __float_as_uint(r0.w), geom = __float_as_uint(r1.w);
             if (t < s.best.t || geom < s.best.geom ||
                 (geom == s.best.geom &&
@@ -676,7 +682,7 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
         }
         if (s.ngroup.y <= 0x00FFFFFFu) {
             if (TWO_LEVEL && s.inst != kNoInst && s.sp() == s.inst_sp) exit_instance(s);
-            if (s.sp() == s.floor()) return true;
+            if (s.at_floor()) return true;
             s.pop_sp();
             s.ngroup = st(s.sp());
         }
@@ -778,7 +784,7 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     if (donor && __popc(m_donor & below) < pairs) {
         e = st(s.floor());
         top = TWO_LEVEL && s.inst != kNoInst && s.floor() < s.inst_sp;
-        s.aux += 1u;
+        s.aux += 1u << 24;
     }
     const uint32_t r = __popc(m_idle & below);
     const bool take = idle && r < pairs;
