@@ -147,16 +147,19 @@ struct RayPre {
     // instance mask in bits 16-23 and the stack depth in bits 24-31; bit 7 marks a first-hit ray
     // among closest-hit ones (kRayAny).
     uint32_t k;
-    float Sx, Sy, Sz;
-    float ox, oy, oz; // origin permuted to (kx, ky, kz)
     GBPT_DI int kx() const { return (int)(k & 3u); }
     GBPT_DI int ky() const { return (int)((k >> 2) & 3u); }
     GBPT_DI int kz() const { return (int)((k >> 4) & 3u); }
     GBPT_DI uint32_t oct_inv() const { return (k >> 8) & 7u; }
     GBPT_DI uint32_t mask() const { return (k >> 16) & 0xFFu; }
 };
+// The rest of the test's ray: the shear, and the origin permuted to (kx, ky, kz).
+struct RayShear {
+    float Sx, Sy, Sz;
+    float ox, oy, oz;
+};
 GBPT_DI float pick(float x, float y, float z, int k) { return k == 0 ? x : (k == 1 ? y : z); }
-GBPT_DI RayPre ray_pre(float3 o, float3 d) {
+GBPT_DI RayPre ray_pre(float3 o, float3 d, RayShear& r) {
     RayPre p;
     const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     const int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
@@ -164,12 +167,12 @@ GBPT_DI RayPre ray_pre(float3 o, float3 d) {
     const int ky = kx == 2 ? 0 : kx + 1;
     const float dkz = pick(d.x, d.y, d.z, kz);
     p.k = (uint32_t)kx | ((uint32_t)ky << 2) | ((uint32_t)kz << 4) | (dkz < 0.0f ? 64u : 0u);
-    p.Sx = __fdiv_rn(pick(d.x, d.y, d.z, kx), dkz);
-    p.Sy = __fdiv_rn(pick(d.x, d.y, d.z, ky), dkz);
-    p.Sz = __frcp_rn(dkz);
-    p.ox = pick(o.x, o.y, o.z, kx);
-    p.oy = pick(o.x, o.y, o.z, ky);
-    p.oz = pick(o.x, o.y, o.z, kz);
+    r.Sx = __fdiv_rn(pick(d.x, d.y, d.z, kx), dkz);
+    r.Sy = __fdiv_rn(pick(d.x, d.y, d.z, ky), dkz);
+    r.Sz = __frcp_rn(dkz);
+    r.ox = pick(o.x, o.y, o.z, kx);
+    r.oy = pick(o.x, o.y, o.z, ky);
+    r.oz = pick(o.x, o.y, o.z, kz);
     return p;
 }
 
@@ -179,38 +182,38 @@ GBPT_DI RayPre ray_pre(float3 o, float3 d) {
 #ifndef GBPT_DEFER_UV
 #define GBPT_DEFER_UV 1
 #endif
-GBPT_DI bool intersect_tri(const RayPre& p, float4 a4, float4 b4, float4 c4, uint32_t tflags,
-                           float tmin, float tmax, float& t_out, float& u_out, float& v_out,
-                           float& det_out) {
+GBPT_DI bool intersect_tri(const RayPre& p, const RayShear& r, float4 a4, float4 b4, float4 c4,
+                           uint32_t tflags, float tmin, float tmax, float& t_out, float& u_out,
+                           float& v_out, float& det_out) {
 #if GBPT_TRI_AXIS_COPIES
     // the record copy of axis kz holds the coordinates (kx, ky, kz)
-    const float Akx = __fsub_rn(a4.x, p.ox);
-    const float Aky = __fsub_rn(a4.y, p.oy);
-    const float Akz = __fsub_rn(a4.z, p.oz);
-    const float Bkx = __fsub_rn(b4.x, p.ox);
-    const float Bky = __fsub_rn(b4.y, p.oy);
-    const float Bkz = __fsub_rn(b4.z, p.oz);
-    const float Ckx = __fsub_rn(c4.x, p.ox);
-    const float Cky = __fsub_rn(c4.y, p.oy);
-    const float Ckz = __fsub_rn(c4.z, p.oz);
+    const float Akx = __fsub_rn(a4.x, r.ox);
+    const float Aky = __fsub_rn(a4.y, r.oy);
+    const float Akz = __fsub_rn(a4.z, r.oz);
+    const float Bkx = __fsub_rn(b4.x, r.ox);
+    const float Bky = __fsub_rn(b4.y, r.oy);
+    const float Bkz = __fsub_rn(b4.z, r.oz);
+    const float Ckx = __fsub_rn(c4.x, r.ox);
+    const float Cky = __fsub_rn(c4.y, r.oy);
+    const float Ckz = __fsub_rn(c4.z, r.oz);
 #else
     const int kx = p.kx(), ky = p.ky(), kz = p.kz();
-    const float Akx = __fsub_rn(pick(a4.x, a4.y, a4.z, kx), p.ox);
-    const float Aky = __fsub_rn(pick(a4.x, a4.y, a4.z, ky), p.oy);
-    const float Akz = __fsub_rn(pick(a4.x, a4.y, a4.z, kz), p.oz);
-    const float Bkx = __fsub_rn(pick(b4.x, b4.y, b4.z, kx), p.ox);
-    const float Bky = __fsub_rn(pick(b4.x, b4.y, b4.z, ky), p.oy);
-    const float Bkz = __fsub_rn(pick(b4.x, b4.y, b4.z, kz), p.oz);
-    const float Ckx = __fsub_rn(pick(c4.x, c4.y, c4.z, kx), p.ox);
-    const float Cky = __fsub_rn(pick(c4.x, c4.y, c4.z, ky), p.oy);
-    const float Ckz = __fsub_rn(pick(c4.x, c4.y, c4.z, kz), p.oz);
+    const float Akx = __fsub_rn(pick(a4.x, a4.y, a4.z, kx), r.ox);
+    const float Aky = __fsub_rn(pick(a4.x, a4.y, a4.z, ky), r.oy);
+    const float Akz = __fsub_rn(pick(a4.x, a4.y, a4.z, kz), r.oz);
+    const float Bkx = __fsub_rn(pick(b4.x, b4.y, b4.z, kx), r.ox);
+    const float Bky = __fsub_rn(pick(b4.x, b4.y, b4.z, ky), r.oy);
+    const float Bkz = __fsub_rn(pick(b4.x, b4.y, b4.z, kz), r.oz);
+    const float Ckx = __fsub_rn(pick(c4.x, c4.y, c4.z, kx), r.ox);
+    const float Cky = __fsub_rn(pick(c4.x, c4.y, c4.z, ky), r.oy);
+    const float Ckz = __fsub_rn(pick(c4.x, c4.y, c4.z, kz), r.oz);
 #endif
-    const float Ax = __fsub_rn(Akx, __fmul_rn(p.Sx, Akz));
-    const float Ay = __fsub_rn(Aky, __fmul_rn(p.Sy, Akz));
-    const float Bx = __fsub_rn(Bkx, __fmul_rn(p.Sx, Bkz));
-    const float By = __fsub_rn(Bky, __fmul_rn(p.Sy, Bkz));
-    const float Cx = __fsub_rn(Ckx, __fmul_rn(p.Sx, Ckz));
-    const float Cy = __fsub_rn(Cky, __fmul_rn(p.Sy, Ckz));
+    const float Ax = __fsub_rn(Akx, __fmul_rn(r.Sx, Akz));
+    const float Ay = __fsub_rn(Aky, __fmul_rn(r.Sy, Akz));
+    const float Bx = __fsub_rn(Bkx, __fmul_rn(r.Sx, Bkz));
+    const float By = __fsub_rn(Bky, __fmul_rn(r.Sy, Bkz));
+    const float Cx = __fsub_rn(Ckx, __fmul_rn(r.Sx, Ckz));
+    const float Cy = __fsub_rn(Cky, __fmul_rn(r.Sy, Ckz));
     float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
     float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
     float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
@@ -226,9 +229,9 @@ GBPT_DI bool intersect_tri(const RayPre& p, float4 a4, float4 b4, float4 c4, uin
         const bool front = (det > 0.0f) != ((p.k & 64u) != 0u);
         if (front == ((tflags & kTriFlip) != 0)) return false;
     }
-    const float Az = __fmul_rn(p.Sz, Akz);
-    const float Bz = __fmul_rn(p.Sz, Bkz);
-    const float Cz = __fmul_rn(p.Sz, Ckz);
+    const float Az = __fmul_rn(r.Sz, Akz);
+    const float Bz = __fmul_rn(r.Sz, Bkz);
+    const float Cz = __fmul_rn(r.Sz, Ckz);
     const float T = __fadd_rn(__fadd_rn(__fmul_rn(U, Az), __fmul_rn(V, Bz)), __fmul_rn(W, Cz));
     const float t = __fdiv_rn(T, det);
     if (!(t >= tmin && t <= tmax)) return false;
@@ -257,6 +260,7 @@ GBPT_DI bool intersect_tri(const RayPre& p, float4 a4, float4 b4, float4 c4, uin
 constexpr int kStackSize = GBPT_STACK_SIZE;
 static_assert(kStackSize >= 1, "the traversal needs a stack entry");
 constexpr uint32_t kNoInst = 0xFFFFFFFFu;
+constexpr int kTraceThreads = 128; // block of every traversal kernel
 
 // Work of the instrumented traversal (COUNT): nodes visited and triangles tested per lane, and
 // on the first active lane of each warp-wide step the step and its active lanes.
@@ -307,6 +311,26 @@ GBPT_DI float3 xform_vector(float4 r0, float4 r1, float4 r2, float3 v) {
 // million closest hits 0.82 / 0.75 / 0.72 ms).
 
 
+// What a node step does not touch, in shared memory: the closest hit (written when a candidate is
+// accepted, two or three times a ray) and the triangle test's ray (read while the triangle's
+// record is on its way). In registers these words made the traversal spill others, 96 to 136 bytes
+// a thread at 8 and 9 blocks per SM, and what it spilled missed L1 two times in three; now it
+// spills 8 to 48 (640x360 soup frame 7.18 instead of 7.35 ms, 1080p 226.1 instead of 227.4, 37,003
+// listed pixels 1.50 instead of 1.55, a million closest hits 0.645 instead of 0.652).
+// 13 words, an odd stride: the lanes' words fall into different banks.
+struct LaneMem {
+    RayShear ray;
+    float u, v, det; // GBPT_DEFER_UV: u, v are V, W of the test until divided by det
+    uint32_t prim, geom, inst; // geom = kNoInst until a hit is found
+    uint32_t pad;
+};
+// The world ray of two-level scenes, read when an instance is entered or left, there as well: it
+// makes room for an eighth block per SM (trace_blocks).
+struct WorldRay {
+    float ox, oy, oz, dx, dy, dz;
+    uint32_t pad;
+};
+
 struct TraceState {
     const uint4* nodes;  // the ray's scene (rays of one launch may belong to different scenes)
     const float4* tris;  // the records (copy-major layout: the current ray's copy)
@@ -317,9 +341,9 @@ struct TraceState {
     float tmin;
     RayPre pre;
     uint2 ngroup, tgroup;
-    Hit best;          // a hit was found once best.geom != kNoInst
-    float det;         // GBPT_DEFER_UV: best.u, best.v are V, W of the test until divided by it
-    float3 wo, wd; // the world ray
+    LaneMem* lane;   // the rest of the closest hit and of the current ray
+    float t; // the closest hit's distance, the span's end before the first
+    WorldRay* world; // of two-level scenes
     uint32_t inst; // instance being traversed, kNoInst at the top level
     int inst_sp;   // stack depth at which it was entered
     // bits 24-31: the stack's first entry of this lane (those below were given to other lanes), as
@@ -368,7 +392,7 @@ GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
                          ((__float_as_uint(d.z) >> 31) << 2);
     // the stack, the mask and the hit outlive a change of space
     const uint32_t kept = s.pre.k & (0xFFFF0000u | kTriKey | kRayAny);
-    s.pre = ray_pre(o, d);
+    s.pre = ray_pre(o, d, s.lane->ray);
     s.pre.k |= ((7u - oct) << 8) | kept;
     s.tris = kTriCopies > 1 ? s.tris_base + (size_t)s.pre.kz() * s.tri_stride : s.tris_base;
 }
@@ -377,17 +401,15 @@ GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tma
                         uint32_t any = 0u) {
     s.pre.k = ((mask & 0xFFu) << 16) | any; // any: kRayAny or 0
     set_ray(s, o, d);
-    s.wo = o;
-    s.wd = d;
     // a span with a NaN end holds no hit, but would make every box test one: an empty span
     const bool span = tmin == tmin && tmax == tmax;
     if (!span) tmin = 0.0f, tmax = -1.0f;
     s.ngroup = make_uint2(0u, 0x80000000u);
     s.tgroup = make_uint2(0u, 0u);
     s.tmin = tmin;
-    s.best.t = tmax;
-    s.best.u = s.best.v = 0.0f;
-    s.best.prim = s.best.geom = s.best.inst = kNoInst;
+    s.t = tmax;
+    s.lane->u = s.lane->v = 0.0f;
+    s.lane->prim = s.lane->geom = s.lane->inst = kNoInst;
     s.inst = kNoInst;
     s.inst_sp = -1;
 }
@@ -395,14 +417,17 @@ GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tma
 GBPT_DI void enter_instance(TraceState& s, const float4* insts, uint32_t ii) {
     const float4* r = insts + 7ull * ii;
     const float4 w0 = __ldg(r + 3), w1 = __ldg(r + 4), w2 = __ldg(r + 5);
-    set_ray(s, xform_point(w0, w1, w2, s.wo), xform_vector(w0, w1, w2, s.wd));
+    const WorldRay& w = *s.world;
+    set_ray(s, xform_point(w0, w1, w2, f3(w.ox, w.oy, w.oz)),
+            xform_vector(w0, w1, w2, f3(w.dx, w.dy, w.dz)));
     s.inst = ii;
     s.inst_sp = s.sp();
     s.ngroup = make_uint2(__float_as_uint(__ldg(r + 6).x), 0x80000000u);
 }
 
 GBPT_DI void exit_instance(TraceState& s) {
-    set_ray(s, s.wo, s.wd);
+    const WorldRay& w = *s.world;
+    set_ray(s, f3(w.ox, w.oy, w.oz), f3(w.dx, w.dy, w.dz));
     s.inst = kNoInst;
     s.inst_sp = -1;
 }
@@ -541,9 +566,9 @@ GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni
                 const float2 tnz = plane_t2<j>(nqz, az2, noz2), tfx = plane_t2<j>(fqx, ax2, fox2);
                 const float2 tfy = plane_t2<j>(fqy, ay2, foy2), tfz = plane_t2<j>(fqz, az2, foz2);
                 const float cmin0 = fmaxf(fmaxf(tnx.x, tny.x), fmaxf(tnz.x, s.tmin));
-                const float cmax0 = fminf(fminf(tfx.x, tfy.x), fminf(tfz.x, s.best.t));
+                const float cmax0 = fminf(fminf(tfx.x, tfy.x), fminf(tfz.x, s.t));
                 const float cmin1 = fmaxf(fmaxf(tnx.y, tny.y), fmaxf(tnz.y, s.tmin));
-                const float cmax1 = fminf(fminf(tfx.y, tfy.y), fminf(tfz.y, s.best.t));
+                const float cmax1 = fminf(fminf(tfx.y, tfy.y), fminf(tfz.y, s.t));
                 add(cmin0, cmax0);
                 add(cmin1, cmax1);
             };
@@ -559,7 +584,7 @@ GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni
                 const float tfy = __fmaf_rn(qplane(fqy, j), aiy, foy);
                 const float tfz = __fmaf_rn(qplane(fqz, j), aiz, foz);
                 const float cmin = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, s.tmin));
-                const float cmax = fminf(fminf(tfx, tfy), fminf(tfz, s.best.t));
+                const float cmax = fminf(fminf(tfx, tfy), fminf(tfz, s.t));
                 add(cmin, cmax);
             }
         }
@@ -579,9 +604,9 @@ GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni
     tgroup = make_uint2(n1.y, tri);
 }
 
-// Runs the traversal of the ray in s until it is finished (returns true; result in s.best, geom
-// = kNoInst on a miss; of a first-hit ray the first hit found) or until the warp should refill its idle
-// lanes (returns false; s keeps the state). `st(i)` is stack entry i. A stack overflow raises *err
+// Runs the traversal of the ray in s until it is finished (returns true; result in s.t and *s.lane,
+// geom = kNoInst on a miss; of a first-hit ray the first hit found) or until the warp should refill
+// its idle lanes (returns false; s keeps the state). `st(i)` is stack entry i. A stack overflow raises *err
 // and finishes the ray with what it found.
 // `alpha(geom, prim, u, v)` decides the candidate hits of non-opaque triangles (true: skip).
 template <TraceMode MODE, bool COUNT, bool TWO_LEVEL, class Scene, class StackRef, class Alpha>
@@ -651,29 +676,30 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             }
             float t, u, v;
             float det;
-            if (!intersect_tri(s.pre, r0, r1, r2, tfl, s.tmin, s.best.t, t, u, v, det)) continue;
+            if (!intersect_tri(s.pre, s.lane->ray, r0, r1, r2, tfl, s.tmin, s.t, t, u, v, det))
+                continue;
             // the instance mask is tested where few candidates get: before the intersection, it made
             // every triangle step wait for the flag word and branch once more (1080p soup frame
             // 235.1 instead of 227.7 ms, a million closest hits 0.72 instead of 0.65). What is
             // counted is still what passes the mask.
             if (!COUNT && (tfl & s.pre.mask()) == 0u) continue;
             const uint32_t prim = __float_as_uint(r0.w), geom = __float_as_uint(r1.w);
-            if (t < s.best.t || geom < s.best.geom ||
-                (geom == s.best.geom &&
-                 (prim < s.best.prim || (prim == s.best.prim && s.inst < s.best.inst)))) {
+            if (t < s.t || geom < s.lane->geom ||
+                (geom == s.lane->geom &&
+                 (prim < s.lane->prim || (prim == s.lane->prim && s.inst < s.lane->inst)))) {
 #if GBPT_DEFER_UV
                 if ((tfl & kTriAlpha) && alpha(geom, prim, __fdiv_rn(u, det), __fdiv_rn(v, det)))
                     continue;
-                s.det = det;
+                s.lane->det = det;
 #else
                 if ((tfl & kTriAlpha) && alpha(geom, prim, u, v)) continue;
 #endif
-                s.best.t = t;
-                s.best.u = u;
-                s.best.v = v;
-                s.best.prim = prim;
-                s.best.geom = geom;
-                s.best.inst = s.inst;
+                s.t = t;
+                s.lane->u = u;
+                s.lane->v = v;
+                s.lane->prim = prim;
+                s.lane->geom = geom;
+                s.lane->inst = s.inst;
                 if (MODE != kTraceAny) s.pre.k = (s.pre.k & ~kTriKey) | (tfl & kTriKey);
                 // a first-hit ray ends with it
                 if (MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u))
@@ -708,10 +734,12 @@ template <class T> GBPT_DI T* shfl_ptr(T* p, uint32_t src) {
     return (T*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)p, src);
 }
 
-// Whether hit a comes before b: nearer, or at the same distance the smaller (geometry, primitive,
-// instance).
-GBPT_DI bool hit_before(float t, uint32_t geom, uint32_t prim, uint32_t inst, const Hit& b) {
-    return t < b.t || (t == b.t && (geom < b.geom ||
+// Whether a hit comes before the lane's: nearer, or at the same distance the smaller (geometry,
+// primitive, instance).
+GBPT_DI bool hit_before(float t, uint32_t geom, uint32_t prim, uint32_t inst,
+                        const TraceState& s) {
+    const LaneMem& b = *s.lane;
+    return t < s.t || (t == s.t && (geom < b.geom ||
                                     (geom == b.geom &&
                                      (prim < b.prim || (prim == b.prim && inst < b.inst)))));
 }
@@ -733,35 +761,35 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     const uint32_t lane = threadIdx.x & 31u;
     // helpers' hits, one at a time, to their rays' owners
     const bool helper = s.owner() != lane;
-    uint32_t m = __ballot_sync(0xFFFFFFFFu, helper && s.best.geom != kNoInst);
+    uint32_t m = __ballot_sync(0xFFFFFFFFu, helper && s.lane->geom != kNoInst);
     while (m != 0u) {
         const uint32_t h = __ffs(m) - 1u;
         m &= m - 1u;
         const uint32_t o = __shfl_sync(0xFFFFFFFFu, s.owner(), h);
-        const float t = __shfl_sync(0xFFFFFFFFu, s.best.t, h);
-        const float u = __shfl_sync(0xFFFFFFFFu, s.best.u, h);
-        const float v = __shfl_sync(0xFFFFFFFFu, s.best.v, h);
-        const float det = __shfl_sync(0xFFFFFFFFu, s.det, h);
-        const uint32_t prim = __shfl_sync(0xFFFFFFFFu, s.best.prim, h);
-        const uint32_t geom = __shfl_sync(0xFFFFFFFFu, s.best.geom, h);
-        const uint32_t inst = TWO_LEVEL ? __shfl_sync(0xFFFFFFFFu, s.best.inst, h) : kNoInst;
+        const float t = __shfl_sync(0xFFFFFFFFu, s.t, h);
+        const float u = __shfl_sync(0xFFFFFFFFu, s.lane->u, h);
+        const float v = __shfl_sync(0xFFFFFFFFu, s.lane->v, h);
+        const float det = __shfl_sync(0xFFFFFFFFu, s.lane->det, h);
+        const uint32_t prim = __shfl_sync(0xFFFFFFFFu, s.lane->prim, h);
+        const uint32_t geom = __shfl_sync(0xFFFFFFFFu, s.lane->geom, h);
+        const uint32_t inst = TWO_LEVEL ? __shfl_sync(0xFFFFFFFFu, s.lane->inst, h) : kNoInst;
         const uint32_t k = __shfl_sync(0xFFFFFFFFu, s.pre.k, h);
-        if (lane == o && hit_before(t, geom, prim, inst, s.best)) {
-            s.best.t = t;
-            s.best.u = u;
-            s.best.v = v;
-            s.det = det;
-            s.best.prim = prim;
-            s.best.geom = geom;
-            s.best.inst = inst;
+        if (lane == o && hit_before(t, geom, prim, inst, s)) {
+            s.t = t;
+            s.lane->u = u;
+            s.lane->v = v;
+            s.lane->det = det;
+            s.lane->prim = prim;
+            s.lane->geom = geom;
+            s.lane->inst = inst;
             s.pre.k = (s.pre.k & ~kTriKey) | (k & kTriKey);
         }
-        if (lane == h) s.best.prim = s.best.geom = s.best.inst = kNoInst;
+        if (lane == h) s.lane->prim = s.lane->geom = s.lane->inst = kNoInst;
     }
     // the owner's distance; a first-hit ray ends with its first hit
-    const float t_own = __shfl_sync(0xFFFFFFFFu, s.best.t, s.owner());
-    const uint32_t g_own = __shfl_sync(0xFFFFFFFFu, s.best.geom, s.owner());
-    if (helper) s.best.t = fminf(s.best.t, t_own);
+    const float t_own = __shfl_sync(0xFFFFFFFFu, s.t, s.owner());
+    const uint32_t g_own = __shfl_sync(0xFFFFFFFFu, s.lane->geom, s.owner());
+    if (helper) s.t = fminf(s.t, t_own);
     const bool any =
         MODE == kTraceAny || (MODE == kTraceMixed && (s.pre.k & kRayAny) != 0u);
     if (any && g_own != kNoInst) active = false;
@@ -796,13 +824,9 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     s.o = f3(f(s.o.x), f(s.o.y), f(s.o.z));
     s.inv = f3(f(s.inv.x), f(s.inv.y), f(s.inv.z));
     if (MODE != kTraceMixed) s.tmin = f(s.tmin); // bounce and shadow rays start at 0
-    s.pre.Sx = f(s.pre.Sx);
-    s.pre.Sy = f(s.pre.Sy);
-    s.pre.Sz = f(s.pre.Sz);
-    s.pre.ox = f(s.pre.ox);
-    s.pre.oy = f(s.pre.oy);
-    s.pre.oz = f(s.pre.oz);
-    s.best.t = f(s.best.t);
+    const RayShear q = s.lane->ray;
+    const RayShear shear{f(q.Sx), f(q.Sy), f(q.Sz), f(q.ox), f(q.oy), f(q.oz)};
+    s.t = f(s.t);
     ray = w(ray);
     const uint32_t k = w(s.pre.k), aux = w(s.aux);
     e.x = w(e.x);
@@ -814,18 +838,20 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
             s.tri_stride = w(s.tri_stride);
             s.insts = shfl_ptr(s.insts, src);
         }
-        s.wo = f3(f(s.wo.x), f(s.wo.y), f(s.wo.z));
-        s.wd = f3(f(s.wd.x), f(s.wd.y), f(s.wd.z));
+        const WorldRay q = *s.world;
+        const WorldRay wr{f(q.ox), f(q.oy), f(q.oz), f(q.dx), f(q.dy), f(q.dz), 0u};
+        if (take) *s.world = wr;
         s.inst = w(s.inst);
         restart = w(top ? 1u : 0u) != 0u;
     }
     if (take) {
         active = true;
+        s.lane->ray = shear;
         s.pre.k = k & ~(0xFF000000u | kTriKey); // an empty stack, no hit
         s.aux = aux & 0x1F00u;
         s.ngroup = e;
         s.tgroup = make_uint2(0u, 0u);
-        s.best.prim = s.best.geom = s.best.inst = kNoInst;
+        s.lane->prim = s.lane->geom = s.lane->inst = kNoInst;
         s.inst_sp = TWO_LEVEL && s.inst != kNoInst ? 0 : -1;
         if (TWO_LEVEL && restart) exit_instance(s);
     }
@@ -852,14 +878,23 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
     auto st_ref = [&](int i) -> uint2& { return stack[i]; };
     // the barycentrics are divided once, for the final hit
     auto store = [&](uint32_t i, TraceState& s) {
-        if (s.best.geom != kNoInst) {
-            s.best.u = __fdiv_rn(s.best.u, s.det);
-            s.best.v = __fdiv_rn(s.best.v, s.det);
+        Hit h{s.t, s.lane->u, s.lane->v, s.lane->prim, s.lane->geom, s.lane->inst};
+        if (h.geom != kNoInst) {
+            h.u = __fdiv_rn(h.u, s.lane->det);
+            h.v = __fdiv_rn(h.v, s.lane->det);
         }
-        store_hit(i, s.best, (s.pre.k & kTriKey) >> kTriKeyShift);
+        store_hit(i, h, (s.pre.k & kTriKey) >> kTriKeyShift);
     };
+    __shared__ LaneMem lanes[kTraceThreads];
     TraceState s;
-    s.best.geom = kNoInst;
+    s.lane = &lanes[threadIdx.x];
+    __shared__ WorldRay worlds[TWO_LEVEL ? kTraceThreads : 1];
+    s.world = &worlds[TWO_LEVEL ? threadIdx.x : 0];
+    auto load_ray = [&](uint32_t i) {
+        load(i, s);
+        if (TWO_LEVEL) *s.world = WorldRay{s.o.x, s.o.y, s.o.z, s.d.x, s.d.y, s.d.z, 0u};
+    };
+    s.lane->geom = kNoInst;
     s.aux = lane << 8;
     uint32_t ray = 0xFFFFFFFFu;
     bool active = false, owns = false, pool_empty = false;
@@ -870,7 +905,7 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
             const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * lanes + lane;
             if (lane < lanes && i < n) {
                 ray = i;
-                load(ray, s);
+                load_ray(ray);
                 active = owns = true;
             }
             pool_empty = true;
@@ -890,7 +925,7 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
                     const uint32_t i = base + __popc(want_mask & ((1u << lane) - 1u));
                     if (i < n) {
                         ray = i;
-                        load(ray, s);
+                        load_ray(ray);
                         active = owns = true;
                     } else {
                         exhausted = true;
@@ -917,7 +952,7 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
             if (!SHARE || !pool_empty) {
                 store(ray, s);
                 owns = false;
-                s.best.geom = kNoInst;
+                s.lane->geom = kNoInst;
             }
         }
     }

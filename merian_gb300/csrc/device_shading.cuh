@@ -425,14 +425,14 @@ template <class K> int persistent_grid(K kernel) {
 #define GBPT_TRACE_BLOCKS_PER_SM 8
 #endif
 constexpr int kTraceBlocksPerSM = GBPT_TRACE_BLOCKS_PER_SM;
-// The two-level variants keep the world ray and the instance as well: 7 blocks (72 registers) spill
-// less than 8 and beat them (instanced 1280x720 frame, 8 / 7 / 6 / 5 blocks: 4.36 / 4.25 / 4.30 /
-// 4.35 ms). The others run 8, and 9 in long queues, where the ninth block hides more of the others'
-// waiting than its spills cost (1080p soup frame 235.0 instead of 239.8 ms, 640x360 7.65 instead of
-// 7.80); short queues end with a few rays whose latency the spills add to (37,003 pixels x 8 1.68
-// instead of 1.64).
+// 9 in long queues of single-level scenes, where the ninth block hides more of the others' waiting
+// than its spills cost (1080p soup frame 235.0 instead of 239.8 ms, 640x360 7.65 instead of 7.80; a
+// tenth costs more: 227.7 instead of 226.1); short queues end with a few rays whose latency the
+// spills add to (37,003 pixels x 8 1.58 instead of 1.50). The two-level variants hold the instance
+// as well and spilled at 8 blocks until the world ray moved to shared memory; now 8 beat 7
+// (instanced 1280x720 frame 3.56 instead of 3.62 ms, its G-buffer 0.757 instead of 0.766).
 constexpr int trace_blocks(bool two_level, bool long_queue = false) {
-    return two_level ? kTraceBlocksPerSM - 1 : kTraceBlocksPerSM + (long_queue ? 1 : 0);
+    return kTraceBlocksPerSM + (long_queue && !two_level ? 1 : 0);
 }
 
 } // namespace gbpt

@@ -43,7 +43,7 @@ GBPT_DI OneScene one_scene(const DevScene& sc) {
 // soup take 0.85 instead of 1.19 ms, 250,000 occlusion rays in the tessellated room 0.15 instead
 // of 0.33.
 template <bool ANY, bool COUNT, bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
+__global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
     k_trace_rays(DevScene sc, const gbpt_ray* rays, uint32_t n, uint32_t mask, gbpt_hit* hits,
                  unsigned long long* work_ctr, uint32_t* fetch, uint32_t* err, int refill_lanes) {
     TraceCounters ctr{0, 0, 0, 0, 0, 0};
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
 // its longest ray was done: the 1920x1080 G-buffer of the instanced scene took 2.43 instead of
 // 0.94 ms.
 template <bool TWO_LEVEL, bool ALPHA>
-__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
+__global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
     k_trace_primary(DevScene sc, CamGPU cam, uint32_t w, uint32_t h, uint32_t mask, gbpt_hit* hits,
                     gbpt_gbuffer_texel* texels, uint32_t* fetch, uint32_t* err, int refill_lanes) {
     auto load = [&](uint32_t i, TraceState& s) {
@@ -200,7 +200,7 @@ int trace_rays(const SceneGPU& scene, const gbpt_ray* rays, uint32_t n, uint32_t
     auto go = [&](auto kernel) {
         int grid = persistent_grid(kernel);
         if (sched.blocks_per_sm) grid = std::min(grid, (int)sched.blocks_per_sm * num_sms());
-        kernel<<<grid, 128, 0, st>>>(sc, rays, n, mask & 0xFFu, hits, work_ctr, fetch, err,
+        kernel<<<grid, kTraceThreads, 0, st>>>(sc, rays, n, mask & 0xFFu, hits, work_ctr, fetch, err,
                                      (int)sched.refill_lanes);
     };
     if (count) {
@@ -230,7 +230,7 @@ void launch_trace_primary(const SceneGPU& scene, const DevScene& sc, const CamGP
     auto go = [&](auto kernel) {
         int grid = std::min(persistent_grid(kernel), (int)(((uint64_t)w * h + 127) / 128));
         if (sched.blocks_per_sm) grid = std::min(grid, (int)sched.blocks_per_sm * num_sms());
-        kernel<<<grid, 128, 0, st>>>(sc, cam, w, h, mask & 0xFFu, hits, texels, fetch, err,
+        kernel<<<grid, kTraceThreads, 0, st>>>(sc, cam, w, h, mask & 0xFFu, hits, texels, fetch, err,
                                      (int)sched.refill_lanes);
     };
     switch ((sc.n_inst ? 2 : 0) | (scene.alpha ? 1 : 0)) {

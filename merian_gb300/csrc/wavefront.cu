@@ -168,7 +168,7 @@ GBPT_DI const ChunkGPU& slot_ray(const TickArgs& t, uint32_t nc, uint32_t q, flo
 // instanced 1280x720 frame 1.80 instead of 0.36 ms, of the 640x360 soup frame 0.54 instead of
 // 0.21 ms; the frames 8.84 instead of 7.47 and 12.42 instead of 12.11 ms).
 template <bool TWO_LEVEL, bool ALPHA, class Scene>
-__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL))
+__global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
     k_trace_pixels(TickArgs t, Scene scene) {
     wait_for_predecessor();
     const uint32_t n = t.hdr->n_pix, nc = t.hdr->n_chunks;
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
 // 640x360 soup frame 8.6 instead of 9.4; the clears of the counters, now one per tick instead of
 // four per vertex, included).
 template <bool COUNT, bool TWO_LEVEL, bool ALPHA, class Scene, bool LONG = false>
-__global__ void __launch_bounds__(128, trace_blocks(TWO_LEVEL, LONG))
+__global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL, LONG))
     k_trace(TickArgs t, Scene scene, int k, int qi, int parts, unsigned long long* work_ctr,
             int sort) {
     wait_for_predecessor();
@@ -961,7 +961,7 @@ void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k,
     const int gr = work_ctr ? g.trace_c : tp.two_level ? g.trace2 : lng ? g.trace_l : g.trace;
     const int so = sort ? 1 : 0;
     auto go = [&](auto kernel, auto scene) {
-        launch(kernel, gr, 128, st, ta, scene, k, qi, parts, work_ctr, so);
+        launch(kernel, gr, kTraceThreads, st, ta, scene, k, qi, parts, work_ctr, so);
     };
     const OneScene one{tp.scene};
     if (tp.one_scene && !work_ctr) {
@@ -988,7 +988,7 @@ void launch_trace(const TickArgs& ta, const TickPlan& tp, const Grids& g, int k,
 
 void launch_trace_pixels(const TickArgs& ta, const TickPlan& tp, int grid, cudaStream_t st) {
     const OneScene one{tp.scene};
-    auto go = [&](auto kernel, auto scene) { launch(kernel, grid, 128, st, ta, scene); };
+    auto go = [&](auto kernel, auto scene) { launch(kernel, grid, kTraceThreads, st, ta, scene); };
     if (tp.one_scene) {
         if (tp.alpha) go(k_trace_pixels<true, true, OneScene>, one);
         else go(k_trace_pixels<true, false, OneScene>, one);
