@@ -397,7 +397,7 @@ def run_gbpt(args):
     ms = float(np.mean(step_ms))
 
     # untimed instrumented pass: CWBVH nodes / triangles per closest-hit ray of this workload by
-    # the kernel's own counters (with its postponed triangle groups)
+    # the kernel's own counters
     ctx.set_profiling(2)
     cst = ctx.render_device(sid, cam, params(frame_base + 999), out.data_ptr(), stats=True)
     kernel_nodes_per_ray = cst.nodes_visited / max(cst.trace_rays, 1)

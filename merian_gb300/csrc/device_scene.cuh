@@ -363,7 +363,7 @@ struct TraceState {
 // ticks), or, when all rays are of one scene, in the kernel's arguments. The latter saves the
 // two-level state five registers (instanced 1280x720 frame 4.09 instead of 4.25 ms; its G-buffer
 // 0.86 instead of 0.90) and the ray queries' two (a million closest hits 0.81 instead of 0.86);
-// the single-level wavefront is no faster with it (1080p soup frame 253.4 against 251.8 ms).
+// the single-level wavefront is no faster with it (1080p soup frame 225.0 against 224.6 ms).
 struct SceneRef {
     const uint4* nodes;
     const float4* tris;
