@@ -331,12 +331,17 @@ struct WorldRay {
     uint32_t pad;
 };
 
-struct TraceState {
-    const uint4* nodes;  // the ray's scene (rays of one launch may belong to different scenes)
-    const float4* tris;  // the records (copy-major layout: the current ray's copy)
-    const float4* tris_base; // copy 0 of the records and the float4 from one copy to the next
-    uint32_t tri_stride;
+// A scene's traversal data.
+struct SceneRef {
+    const uint4* nodes;
+    const float4* tris;  // copy 0 of the records
     const float4* insts; // instance records; nullptr for single-level scenes
+    uint32_t tri_stride; // float4 from one copy of the records to the next
+};
+
+struct TraceState {
+    SceneRef ref;        // the ray's scene (RayScene)
+    const float4* tris;  // its records (copy-major layout: the current ray's copy)
     float3 o, d, inv;    // the ray in the current space (object space inside an instance)
     float tmin;
     RayPre pre;
@@ -364,27 +369,20 @@ struct TraceState {
 // two-level state five registers (instanced 1280x720 frame 4.09 instead of 4.25 ms; its G-buffer
 // 0.86 instead of 0.90) and the ray queries' two (a million closest hits 0.81 instead of 0.86);
 // the single-level wavefront is no faster with it (1080p soup frame 225.0 against 224.6 ms).
-struct SceneRef {
-    const uint4* nodes;
-    const float4* tris;
-    const float4* insts;
-    uint32_t tri_stride;
-};
+// A lane that works on another lane's ray without having loaded one (share_rays) finds OneScene's
+// data there too: nothing of it is in the lane's state.
 struct RayScene {
     static constexpr bool kPerRay = true;
-    GBPT_DI const uint4* nodes(const TraceState& s) const { return s.nodes; }
-    GBPT_DI const float4* tris(const TraceState& s) const { return s.tris; }
-    GBPT_DI const float4* insts(const TraceState& s) const { return s.insts; }
+    GBPT_DI const SceneRef& of(const TraceState& s) const { return s.ref; }
 };
 struct OneScene {
     static constexpr bool kPerRay = false;
     SceneRef ref;
-    GBPT_DI const uint4* nodes(const TraceState&) const { return ref.nodes; }
-    GBPT_DI const float4* tris(const TraceState& s) const { return s.tris; }
-    GBPT_DI const float4* insts(const TraceState&) const { return ref.insts; }
+    GBPT_DI const SceneRef& of(const TraceState&) const { return ref; }
 };
 
-GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
+template <class Scene>
+GBPT_DI void set_ray(TraceState& s, const Scene& scene, float3 o, float3 d) {
     s.o = o;
     s.d = d;
     s.inv = f3(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
@@ -394,13 +392,15 @@ GBPT_DI void set_ray(TraceState& s, float3 o, float3 d) {
     const uint32_t kept = s.pre.k & (0xFFFF0000u | kTriKey | kRayAny);
     s.pre = ray_pre(o, d, s.lane->ray);
     s.pre.k |= ((7u - oct) << 8) | kept;
-    s.tris = kTriCopies > 1 ? s.tris_base + (size_t)s.pre.kz() * s.tri_stride : s.tris_base;
+    const SceneRef& ref = scene.of(s);
+    s.tris = kTriCopies > 1 ? ref.tris + (size_t)s.pre.kz() * ref.tri_stride : ref.tris;
 }
 
-GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tmax, uint32_t mask,
-                        uint32_t any = 0u) {
+template <class Scene>
+GBPT_DI void trace_init(TraceState& s, const Scene& scene, float3 o, float3 d, float tmin,
+                        float tmax, uint32_t mask, uint32_t any = 0u) {
     s.pre.k = ((mask & 0xFFu) << 16) | any; // any: kRayAny or 0
-    set_ray(s, o, d);
+    set_ray(s, scene, o, d);
     // a span with a NaN end holds no hit, but would make every box test one: an empty span
     const bool span = tmin == tmin && tmax == tmax;
     if (!span) tmin = 0.0f, tmax = -1.0f;
@@ -414,20 +414,21 @@ GBPT_DI void trace_init(TraceState& s, float3 o, float3 d, float tmin, float tma
     s.inst_sp = -1;
 }
 
-GBPT_DI void enter_instance(TraceState& s, const float4* insts, uint32_t ii) {
-    const float4* r = insts + 7ull * ii;
+template <class Scene>
+GBPT_DI void enter_instance(TraceState& s, const Scene& scene, uint32_t ii) {
+    const float4* r = scene.of(s).insts + 7ull * ii;
     const float4 w0 = __ldg(r + 3), w1 = __ldg(r + 4), w2 = __ldg(r + 5);
     const WorldRay& w = *s.world;
-    set_ray(s, xform_point(w0, w1, w2, f3(w.ox, w.oy, w.oz)),
+    set_ray(s, scene, xform_point(w0, w1, w2, f3(w.ox, w.oy, w.oz)),
             xform_vector(w0, w1, w2, f3(w.dx, w.dy, w.dz)));
     s.inst = ii;
     s.inst_sp = s.sp();
     s.ngroup = make_uint2(__float_as_uint(__ldg(r + 6).x), 0x80000000u);
 }
 
-GBPT_DI void exit_instance(TraceState& s) {
+template <class Scene> GBPT_DI void exit_instance(TraceState& s, const Scene& scene) {
     const WorldRay& w = *s.world;
-    set_ray(s, f3(w.ox, w.oy, w.oz), f3(w.dx, w.dy, w.dz));
+    set_ray(s, scene, f3(w.ox, w.oy, w.oz), f3(w.dx, w.dy, w.dz));
     s.inst = kNoInst;
     s.inst_sp = -1;
 }
@@ -633,7 +634,7 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             // the paired planes hold more registers: first-hit traversal, which keeps fewer,
             // measured faster with the scalar ones
             intersect_node<COUNT, GBPT_BOX_FMA2 != 0 && MODE != kTraceAny>(
-                s, scene.nodes(s), ni, order, s.ngroup, s.tgroup, ctr);
+                s, scene.of(s).nodes, ni, order, s.ngroup, s.tgroup, ctr);
         } else {
             // the rest of a top-level instance group came off the stack
             s.tgroup = s.ngroup;
@@ -643,9 +644,9 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             const uint32_t b = __ffs(s.tgroup.y) - 1u;
             s.tgroup.y &= s.tgroup.y - 1u;
             const uint32_t ti = s.tgroup.x + b;
-            if (TWO_LEVEL && scene.insts(s) != nullptr && s.inst == kNoInst) {
+            if (TWO_LEVEL && scene.of(s).insts != nullptr && s.inst == kNoInst) {
                 // a top-level leaf: an instance (record: instance index, mask in the flag word)
-                const uint32_t fl = __float_as_uint(__ldg(&scene.tris(s)[3 * ti + 2]).w);
+                const uint32_t fl = __float_as_uint(__ldg(&s.tris[3 * ti + 2]).w);
                 if ((fl & s.pre.mask()) == 0u) continue;
                 if (s.sp() + 2 > kStackSize) {
                     atomicOr(err, 1u);
@@ -661,10 +662,10 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
                     s.push_sp();
                 }
                 s.tgroup.y = 0u;
-                enter_instance(s, scene.insts(s), __float_as_uint(__ldg(&scene.tris(s)[3 * ti]).w));
+                enter_instance(s, scene, __float_as_uint(__ldg(&s.tris[3 * ti]).w));
                 break;
             }
-            const float4* rec = scene.tris(s) + 3 * ti;
+            const float4* rec = s.tris + 3 * ti;
             const float4 r0 = __ldg(rec + 0);
             const float4 r1 = __ldg(rec + 1);
             const float4 r2 = __ldg(rec + 2);
@@ -707,7 +708,7 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             }
         }
         if (s.ngroup.y <= 0x00FFFFFFu) {
-            if (TWO_LEVEL && s.inst != kNoInst && s.sp() == s.inst_sp) exit_instance(s);
+            if (TWO_LEVEL && s.inst != kNoInst && s.sp() == s.inst_sp) exit_instance(s, scene);
             if (s.at_floor()) return true;
             s.pop_sp();
             s.ngroup = st(s.sp());
@@ -755,8 +756,8 @@ GBPT_DI bool hit_before(float t, uint32_t geom, uint32_t prim, uint32_t inst,
 // frame of path length 16 takes 5.56 / 4.41 ms, 37,003 pixels x 8 of the 200k-triangle soup 2.17 /
 // 1.79, a 64x64 frame of the room 0.30 / 0.25; where queues are long it is neutral (1080p soup
 // frame 261.5 / 260.6).
-template <TraceMode MODE, bool TWO_LEVEL, bool PER_RAY, class StackRef, class Store>
-GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& active, bool& owns,
+template <TraceMode MODE, bool TWO_LEVEL, class Scene, class StackRef, class Store>
+GBPT_DI void share_rays(TraceState& s, const Scene& scene, StackRef&& st, uint32_t& ray, bool& active, bool& owns,
                         const Store& store) {
     const uint32_t lane = threadIdx.x & 31u;
     // helpers' hits, one at a time, to their rays' owners
@@ -819,7 +820,7 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     const uint32_t src = take ? nth_bit(m_donor, r) : lane;
     auto f = [&](float x) { return __shfl_sync(0xFFFFFFFFu, x, src); };
     auto w = [&](uint32_t x) { return __shfl_sync(0xFFFFFFFFu, x, src); };
-    if (PER_RAY) s.nodes = shfl_ptr(s.nodes, src);
+    if (Scene::kPerRay) s.ref.nodes = shfl_ptr(s.ref.nodes, src);
     s.tris = shfl_ptr(s.tris, src);
     s.o = f3(f(s.o.x), f(s.o.y), f(s.o.z));
     s.inv = f3(f(s.inv.x), f(s.inv.y), f(s.inv.z));
@@ -833,10 +834,10 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
     e.y = w(e.y);
     bool restart = false;
     if (TWO_LEVEL) {
-        if (PER_RAY) {
-            s.tris_base = shfl_ptr(s.tris_base, src);
-            s.tri_stride = w(s.tri_stride);
-            s.insts = shfl_ptr(s.insts, src);
+        if (Scene::kPerRay) {
+            s.ref.tris = shfl_ptr(s.ref.tris, src);
+            s.ref.tri_stride = w(s.ref.tri_stride);
+            s.ref.insts = shfl_ptr(s.ref.insts, src);
         }
         const WorldRay q = *s.world;
         const WorldRay wr{f(q.ox), f(q.oy), f(q.oz), f(q.dx), f(q.dy), f(q.dz), 0u};
@@ -853,13 +854,13 @@ GBPT_DI void share_rays(TraceState& s, StackRef&& st, uint32_t& ray, bool& activ
         s.tgroup = make_uint2(0u, 0u);
         s.lane->prim = s.lane->geom = s.lane->inst = kNoInst;
         s.inst_sp = TWO_LEVEL && s.inst != kNoInst ? 0 : -1;
-        if (TWO_LEVEL && restart) exit_instance(s);
+        if (TWO_LEVEL && restart) exit_instance(s, scene);
     }
 }
 
 // Runs the traversal of every ray i < n with persistent warps that pull ray indices from *fetch
 // (zero before the launch; one atomic per warp for all idle lanes). load(i, state) calls
-// trace_init and, when `scene` is per ray, sets ray i's scene (nodes, tris, insts) before; store(i, hit, key) receives its result
+// trace_init and, when `scene` is per ray, sets ray i's scene (s.ref) before; store(i, hit, key) receives its result
 // and the material-sort key of the closest hit (0 on a miss);
 // alpha(i, geom, prim, u, v) is ray i's alpha test (true: skip the candidate). Must be called by
 // all 32 lanes of every warp. Fewer rays than lanes are spread over all warps, a few lanes of
@@ -886,7 +887,12 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
         store_hit(i, h, (s.pre.k & kTriKey) >> kTriKeyShift);
     };
     __shared__ LaneMem lanes[kTraceThreads];
-    TraceState s;
+    // a lane that has not loaded a ray may help with another's, and what share_rays does not hand
+    // over (tmin of bounce and shadow rays, the instance of a single-level scene) is then this
+    // initial state: the values that every load sets, which keep them constants
+    TraceState s{};
+    s.inst = kNoInst;
+    s.inst_sp = -1;
     s.lane = &lanes[threadIdx.x];
     __shared__ WorldRay worlds[TWO_LEVEL ? kTraceThreads : 1];
     s.world = &worlds[TWO_LEVEL ? threadIdx.x : 0];
@@ -934,7 +940,7 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
                 pool_empty = __ballot_sync(0xFFFFFFFFu, exhausted) != 0u;
             }
         }
-        if (SHARE && pool_empty) share_rays<MODE, TWO_LEVEL, Scene::kPerRay>(s, st_ref, ray, active, owns, store);
+        if (SHARE && pool_empty) share_rays<MODE, TWO_LEVEL>(s, scene, st_ref, ray, active, owns, store);
         if (__ballot_sync(0xFFFFFFFFu, active) == 0u) {
             if (!SHARE || __ballot_sync(0xFFFFFFFFu, owns) == 0u) break;
             continue;

@@ -47,11 +47,10 @@ __global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
     k_trace_rays(DevScene sc, const gbpt_ray* rays, uint32_t n, uint32_t mask, gbpt_hit* hits,
                  unsigned long long* work_ctr, uint32_t* fetch, uint32_t* err, int refill_lanes) {
     TraceCounters ctr{0, 0, 0, 0, 0, 0};
+    const OneScene scene = one_scene(sc);
     auto load = [&](uint32_t i, TraceState& s) {
         const gbpt_ray r = rays[i];
-        s.tris_base = sc.tris;
-        s.tri_stride = sc.tri_stride;
-        trace_init(s, f3(r.origin[0], r.origin[1], r.origin[2]),
+        trace_init(s, scene, f3(r.origin[0], r.origin[1], r.origin[2]),
                    f3(r.direction[0], r.direction[1], r.direction[2]), r.tmin, r.tmax, mask);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t) { hits[i] = to_hit(sc, h); };
@@ -59,7 +58,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
     trace_persistent<ANY ? kTraceAny : kTraceClosest, COUNT, TWO_LEVEL, !ANY && !COUNT>(
-        one_scene(sc), n, fetch, load, store, alpha, &ctr, err, refill_lanes);
+        scene, n, fetch, load, store, alpha, &ctr, err, refill_lanes);
     if (COUNT) {
         atomicAdd(work_ctr + 0, (unsigned long long)ctr.nodes);
         atomicAdd(work_ctr + 1, (unsigned long long)ctr.tris);
@@ -76,13 +75,12 @@ template <bool TWO_LEVEL, bool ALPHA>
 __global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
     k_trace_primary(DevScene sc, CamGPU cam, uint32_t w, uint32_t h, uint32_t mask, gbpt_hit* hits,
                     gbpt_gbuffer_texel* texels, uint32_t* fetch, uint32_t* err, int refill_lanes) {
+    const OneScene scene = one_scene(sc);
     auto load = [&](uint32_t i, TraceState& s) {
         float3 o, d;
         float tmin, tmax;
         camera_ray(cam, i % w, i / w, w, h, o, d, tmin, tmax);
-        s.tris_base = sc.tris;
-        s.tri_stride = sc.tri_stride;
-        trace_init(s, o, d, tmin, tmax, mask);
+        trace_init(s, scene, o, d, tmin, tmax, mask);
     };
     auto store = [&](uint32_t i, const Hit& ht, uint32_t) {
         if (!texels) {
@@ -101,7 +99,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
         return ALPHA && alpha_discard(sc, g, p, u, v);
     };
     trace_persistent<kTraceClosest, false, TWO_LEVEL, true>(
-        one_scene(sc), w * h, fetch, load, store, alpha, nullptr, err, refill_lanes);
+        scene, w * h, fetch, load, store, alpha, nullptr, err, refill_lanes);
 }
 
 GBPT_DI uint32_t pack_half2_rn(float lo, float hi) {

@@ -176,16 +176,8 @@ __global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL))
         float3 o, d;
         float tmin, tmax;
         const ChunkGPU& c = slot_ray(t, nc, i, o, d, tmin, tmax);
-        if constexpr (Scene::kPerRay) {
-            s.nodes = c.nodes;
-            s.tris_base = c.tris;
-            s.tri_stride = c.tri_stride;
-            s.insts = c.insts;
-        } else {
-            s.tris_base = scene.ref.tris;
-            s.tri_stride = scene.ref.tri_stride;
-        }
-        trace_init(s, o, d, tmin, tmax, c.mask);
+        if (Scene::kPerRay) s.ref = SceneRef{c.nodes, c.tris, c.insts, c.tri_stride};
+        trace_init(s, scene, o, d, tmin, tmax, c.mask);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t) { store_hit(t.w.hit, i, h); };
     auto alpha = [&](uint32_t i, uint32_t g, uint32_t p, float u, float v) {
@@ -442,17 +434,9 @@ __global__ void __launch_bounds__(kTraceThreads, trace_blocks(TWO_LEVEL, LONG))
         const float4 a = e[0], b = e[1];
         const uint32_t tag = shadow ? __ldg(&t.w.s_path[i - n_rays]) : __float_as_uint(b.w);
         const ChunkGPU& c = t.chunks[tag >> kPathBits];
-        if constexpr (Scene::kPerRay) {
-            s.nodes = c.nodes;
-            s.tris_base = c.tris;
-            s.tri_stride = c.tri_stride;
-            s.insts = c.insts;
-        } else {
-            s.tris_base = scene.ref.tris;
-            s.tri_stride = scene.ref.tri_stride;
-        }
-        trace_init(s, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f, shadow ? a.w : kRayTmax,
-                   c.mask, shadow ? kRayAny : 0u);
+        if (Scene::kPerRay) s.ref = SceneRef{c.nodes, c.tris, c.insts, c.tri_stride};
+        trace_init(s, scene, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), 0.0f,
+                   shadow ? a.w : kRayTmax, c.mask, shadow ? kRayAny : 0u);
     };
     auto store = [&](uint32_t i, const Hit& h, uint32_t key) {
         if (i < n_rays) {
