@@ -396,6 +396,10 @@ GBPT_DI void set_ray(TraceState& s, const Scene& scene, float3 o, float3 d) {
     s.tris = kTriCopies > 1 ? ref.tris + (size_t)s.pre.kz() * ref.tri_stride : ref.tris;
 }
 
+// A span's start with -0 for +0, as intersect_node needs it. (The distance made +0 there instead
+// cost a register: a million closest hits 640 against 626 us.)
+GBPT_DI float span_start(float tmin) { return tmin == 0.0f ? -0.0f : tmin; }
+
 template <class Scene>
 GBPT_DI void trace_init(TraceState& s, const Scene& scene, float3 o, float3 d, float tmin,
                         float tmax, uint32_t mask, uint32_t any = 0u) {
@@ -406,7 +410,7 @@ GBPT_DI void trace_init(TraceState& s, const Scene& scene, float3 o, float3 d, f
     if (!span) tmin = 0.0f, tmax = -1.0f;
     s.ngroup = make_uint2(0u, 0x80000000u);
     s.tgroup = make_uint2(0u, 0u);
-    s.tmin = tmin;
+    s.tmin = span_start(tmin);
     s.t = tmax;
     s.lane->u = s.lane->v = 0.0f;
     s.lane->prim = s.lane->geom = s.lane->inst = kNoInst;
@@ -542,7 +546,11 @@ GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni
     const bool negx = (oct_inv & 1u) == 0u, negy = (oct_inv & 2u) == 0u;
     const bool negz = (oct_inv & 4u) == 0u;
     // the children missed, the first child in the highest bit: the sign of cmax - cmin is set
-    // exactly when cmin <= cmax is false (no NaN gets here: trace_init ends such rays)
+    // when cmin <= cmax is false. Neither is NaN (trace_init ends such rays), and inf - inf is the
+    // canonical, positive NaN. It is also set for cmin = +0 and cmax = -0, the distance of a hit
+    // at the origin along a negative axis (-0 - +0 = -0): so a span never starts at +0
+    // (span_start), and a near plane, which the slack puts before the box, is +0 only where the
+    // box begins beyond 0.
     uint32_t miss = 0;
     auto add = [&](float cmin, float cmax) {
         miss = __funnelshift_l(__float_as_uint(__fsub_rn(cmax, cmin)), miss, 1);
@@ -891,6 +899,7 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
     // over (tmin of bounce and shadow rays, the instance of a single-level scene) is then this
     // initial state: the values that every load sets, which keep them constants
     TraceState s{};
+    s.tmin = span_start(0.0f);
     s.inst = kNoInst;
     s.inst_sp = -1;
     s.lane = &lanes[threadIdx.x];

@@ -1,7 +1,8 @@
 """The device traversal run on the host (traversal_host.cpp): rays shared among a warp's lanes.
 
 Unset lane state holds a pattern and reads outside the scene's arrays are counted, so these tests
-see on the CPU what a helper lane that never loaded a ray of its own works with.
+see on the CPU what a helper lane that never loaded a ray of its own works with. Hits at the
+ray's origin (t = +0 or -0) follow the tie rule here and on the GPU.
 """
 import ctypes as C
 import subprocess
@@ -33,17 +34,16 @@ def _soup():
     return S.soup(n_triangles=4000, n_geometries=8, env_size=None)
 
 
-def _instances():
-    """Eight overlapping instances of one BLAS: translations and a permutation of the axes, whose
-    inverses are exact."""
+def _instances(sc, axes):
+    """Eight overlapping instances of one BLAS: translations by sixteenths and, with `axes`, a
+    permutation of the axes; their inverses are exact."""
     from merian_gb300 import _native as N
     from merian_gb300 import scene as S
-    sc = _soup()
     rng = np.random.default_rng(4)
     inst = np.zeros(8, N.INSTANCE_DTYPE)
     for k in range(8):
         m = np.zeros((3, 4), np.float32)
-        m[:, :3] = np.roll(np.eye(3), k, axis=0)
+        m[:, :3] = np.roll(np.eye(3), k if axes else 0, axis=0)
         m[:, 3] = np.round(rng.uniform(0, 0.75, 3) * 16) / 16
         inst["object_to_world"][k] = m.reshape(inst["object_to_world"][k].shape)
         inst["blas"][k] = 0
@@ -87,7 +87,7 @@ def test_helpers_have_the_state_they_use(host, kind, mode, n, grid):
     no read outside the scene."""
     from merian_gb300 import _native as N
     from merian_gb300 import scene as S
-    sc = _soup() if kind == "single" else _instances()
+    sc = _soup() if kind == "single" else _instances(_soup(), True)
     nodes, tris, _ = S.build_bvh(sc, N.BVH_MEDIUM)
     insts = None
     if kind == "instanced":
@@ -113,3 +113,130 @@ def test_helpers_have_the_state_they_use(host, kind, mode, n, grid):
         assert np.array_equal(h[f][c].view(np.uint32), o[f][c].view(np.uint32)), f
     if kind == "instanced":
         assert np.array_equal(h["instance_id"][c], o["instance_index"][c])
+
+
+def _sheets():
+    """Three sheets of 8 x 8 quads, one perpendicular to each axis, every triangle a two-sided
+    geometry of its own in a random order: a point of a sheet lies in up to six of them."""
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    tris = []
+    for a in range(3):
+        for i in range(8):
+            for j in range(8):
+                q = np.zeros((4, 3))
+                q[:, a] = 2.0 + 3.0 * a
+                q[:, (a + 1) % 3] = np.array([i, i + 1, i + 1, i]) / 8.0
+                q[:, (a + 2) % 3] = np.array([j, j, j + 1, j + 1]) / 8.0
+                tris += [q[[0, 1, 2]], q[[0, 2, 3]]]
+    tris = np.array(tris)[np.random.default_rng(9).permutation(len(tris))]
+    n = len(tris)
+    v = np.zeros(3 * n, N.VERTEX_DTYPE)
+    v["position"] = tris.reshape(-1, 3)
+    g = np.zeros(n, N.GEOMETRY_DTYPE)
+    g["first_triangle"] = np.arange(n)
+    g["triangle_count"] = 1
+    g["flags"] = N.MESH_TWO_SIDED
+    g["instance_mask"] = 0xFF
+    m = np.zeros(1, N.MATERIAL_DTYPE)
+    m["model"] = N.MATERIAL_DIFFUSE
+    m["base_color_texture"] = m["alpha_texture"] = -1
+    return S.SceneData(v, np.arange(3 * n, dtype=np.uint32).reshape(-1, 3), g, m, None), tris
+
+
+def _origin_hits(two_level):
+    """Rays that start on a vertex or an edge of a sheet, along either direction of its axis:
+    (scene, rays, expected geometry, expected instance). The span starts at 0; of some it ends at
+    +0 or -0."""
+    from merian_gb300 import _native as N
+    sc, tris = _sheets()
+    shifts = np.zeros((1, 3))
+    if two_level:
+        sc = _instances(sc, False)
+        shifts = np.array([np.asarray(i["object_to_world"], np.float64).reshape(3, 4)[:, 3]
+                           for i in sc.instances])
+    rng = np.random.default_rng(2)
+    rays, geom, inst = [], [], []
+    for k in range(192):
+        a = k % 3
+        p = np.zeros(3)
+        p[a] = 2.0 + 3.0 * a
+        p[(a + 1) % 3] = rng.integers(0, 9) / 8.0
+        p[(a + 2) % 3] = rng.integers(0, 17) / 16.0
+        s = int(rng.integers(0, len(shifts)))
+        p = p + shifts[s]
+        best = None
+        for i, t in enumerate(shifts):
+            x = p - t
+            if x[a] != 2.0 + 3.0 * a:
+                continue
+            u, w = (a + 1) % 3, (a + 2) % 3
+            c = tris[:, :, [u, w]] - x[[u, w]]
+            area = [c[:, m, 0] * c[:, (m + 1) % 3, 1] - c[:, m, 1] * c[:, (m + 1) % 3, 0]
+                    for m in range(3)]
+            inside = (np.min(area, 0) >= 0) | (np.max(area, 0) <= 0)
+            for j in np.nonzero(inside & (tris[:, 0, a] == x[a]))[0]:
+                best = min(best or (int(j), i), (int(j), i))
+        d = np.zeros(3)
+        d[a] = 1.0 if k % 2 else -1.0
+        if rng.uniform() < 0.7:
+            d[(a + 1) % 3], d[(a + 2) % 3] = rng.uniform(-0.5, 0.5, 2)
+        r = np.zeros(1, N.RAY_DTYPE)
+        r["origin"], r["direction"] = p, d
+        r["tmax"] = [1e7, 1e7, 0.0, -0.0][int(rng.integers(0, 4))]
+        rays.append(r)
+        geom.append(best[0])
+        inst.append(best[1])
+    return sc, np.concatenate(rays), np.array(geom, np.uint32), np.array(inst, np.uint32)
+
+
+@pytest.mark.parametrize("kind", ["single", "instanced"])
+@pytest.mark.parametrize("mode", ["query", "tick of many scenes"])
+@pytest.mark.parametrize("grid", [192, 16, 1])
+def test_hits_at_the_origin(host, kind, mode, grid):
+    """The smallest (geometry, primitive, instance) of the triangles that hold the origin,
+    whatever the sign of t = 0 and the order of the visits."""
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    sc, rays, geom, inst = _origin_hits(kind == "instanced")
+    nodes, tris, _ = S.build_bvh(sc, N.BVH_MEDIUM)
+    insts = None
+    if kind == "instanced":
+        insts = _records(sc, nodes, len(S.build_bvh(_sheets()[0], N.BVH_MEDIUM)[0]))
+    h, bad = _run(host, nodes, tris, insts, rays, np.zeros(len(rays)), mode != "query", 1, grid)
+    assert bad == 0 and (h["t"] == 0).all()
+    assert np.signbit(h["t"]).any() and not np.signbit(h["t"]).all()
+    assert np.array_equal(h["geometry_index"], geom)
+    if kind == "instanced":
+        assert np.array_equal(h["instance_id"], inst)
+    else:
+        w, _ = O.cwbvh_trace(nodes, tris, rays, hit_dtype=N.HIT_DTYPE)
+        assert np.array_equal(w["geometry_index"], geom)
+        assert np.array_equal(w["t"].view(np.uint32), h["t"].view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["single", "instanced"])
+def test_gpu_hits_at_the_origin(gpu_ctx, kind):
+    """The same on the GPU, counting traversal included: few rays (spread over all warps) to more
+    rays than lanes."""
+    import torch
+    from merian_gb300 import _native as N
+    sc, rays, geom, inst = _origin_hits(kind == "instanced")
+    sid = gpu_ctx.upload(sc)
+    try:
+        for n in (1, 192, 5000, 200_000):
+            k = np.arange(n) % len(rays)
+            r = torch.from_numpy(rays[k].view(np.float32).reshape(n, 8)).cuda()
+            h = torch.zeros((n, 8), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            for counted in (False, True):
+                gpu_ctx.trace(sid, r.data_ptr(), n, h.data_ptr(), counted=counted)
+                gpu_ctx.synchronize()
+                g = np.frombuffer(h.cpu().numpy().tobytes(), N.HIT_DTYPE)
+                assert (g["t"] == 0).all()
+                assert np.array_equal(g["geometry_index"], geom[k]), (n, counted)
+                if kind == "instanced":
+                    assert np.array_equal(g["instance_index"], inst[k]), (n, counted)
+    finally:
+        gpu_ctx.destroy_scene(sid)
