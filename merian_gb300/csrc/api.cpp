@@ -577,16 +577,15 @@ GBPT_API int gbpt_scene_create(gbpt_ctx* ctx, const gbpt_scene_desc* d, uint32_t
     for (int k = 1; k <= 3; ++k)
         s.bsdf_kinds += std::find(geom_key.begin(), geom_key.end(), (uint8_t)k) != geom_key.end();
     if ((rc = upload(&s.nodes, bvh.nodes.data(), bvh.nodes.size() * sizeof(CwNode), bytes))) return fail(rc);
-#if GBPT_TRI_AXIS_COPIES
     {
         // three copies of the records, one after the other, coordinates in the order
         // (c + 1, c + 2, c) mod 3 in copy c (the traversal's watertight test reads copy kz)
         // and the material-sort key of the geometry in the flag word (kTriKeyShift)
-        std::vector<TriRecord> rec(3 * bvh.tris.size());
+        std::vector<TriRecord> rec(kTriCopies * bvh.tris.size());
         for (size_t i = 0; i < bvh.tris.size(); ++i) {
             TriRecord r = bvh.tris[i];
             if (r.geom < d->geometry_count) r.pad |= (uint32_t)geom_key[r.geom] << 11;
-            for (int c = 0; c < 3; ++c) {
+            for (int c = 0; c < kTriCopies; ++c) {
                 TriRecord& o = rec[c * bvh.tris.size() + i];
                 o = r;
                 for (int a = 0; a < 3; ++a) {
@@ -599,9 +598,6 @@ GBPT_API int gbpt_scene_create(gbpt_ctx* ctx, const gbpt_scene_desc* d, uint32_t
         }
         if ((rc = upload(&s.tris, rec.data(), rec.size() * sizeof(TriRecord), bytes))) return fail(rc);
     }
-#else
-    if ((rc = upload(&s.tris, bvh.tris.data(), bvh.tris.size() * sizeof(TriRecord), bytes))) return fail(rc);
-#endif
     if ((rc = upload(&s.verts, d->vertices, d->vertex_count * sizeof(gbpt_packed_vertex), bytes))) return fail(rc);
     if ((rc = upload(&s.idx, d->indices, d->triangle_count * 3 * sizeof(uint32_t), bytes))) return fail(rc);
 #if GBPT_SHADE_TRI_RECORDS

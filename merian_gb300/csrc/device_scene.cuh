@@ -147,8 +147,6 @@ struct RayPre {
     // instance mask in bits 16-23 and the stack depth in bits 24-31; bit 7 marks a first-hit ray
     // among closest-hit ones (kRayAny).
     uint32_t k;
-    GBPT_DI int kx() const { return (int)(k & 3u); }
-    GBPT_DI int ky() const { return (int)((k >> 2) & 3u); }
     GBPT_DI int kz() const { return (int)((k >> 4) & 3u); }
     GBPT_DI uint32_t oct_inv() const { return (k >> 8) & 7u; }
     GBPT_DI uint32_t mask() const { return (k >> 16) & 0xFFu; }
@@ -177,15 +175,11 @@ GBPT_DI RayPre ray_pre(float3 o, float3 d, RayShear& r) {
 }
 
 // Returns true with t, u, v when hit within [tmin, tmax] on an accepted face.
-// With GBPT_DEFER_UV the barycentrics are returned undivided (u_out = V, v_out = W, det_out =
-// det): the caller divides them once for the final hit instead of at every accepted candidate.
-#ifndef GBPT_DEFER_UV
-#define GBPT_DEFER_UV 1
-#endif
+// The barycentrics are returned undivided (u_out = V, v_out = W, det_out = det): the caller divides
+// them once for the final hit instead of at every accepted candidate.
 GBPT_DI bool intersect_tri(const RayPre& p, const RayShear& r, float4 a4, float4 b4, float4 c4,
                            uint32_t tflags, float tmin, float tmax, float& t_out, float& u_out,
                            float& v_out, float& det_out) {
-#if GBPT_TRI_AXIS_COPIES
     // the record copy of axis kz holds the coordinates (kx, ky, kz)
     const float Akx = __fsub_rn(a4.x, r.ox);
     const float Aky = __fsub_rn(a4.y, r.oy);
@@ -196,18 +190,6 @@ GBPT_DI bool intersect_tri(const RayPre& p, const RayShear& r, float4 a4, float4
     const float Ckx = __fsub_rn(c4.x, r.ox);
     const float Cky = __fsub_rn(c4.y, r.oy);
     const float Ckz = __fsub_rn(c4.z, r.oz);
-#else
-    const int kx = p.kx(), ky = p.ky(), kz = p.kz();
-    const float Akx = __fsub_rn(pick(a4.x, a4.y, a4.z, kx), r.ox);
-    const float Aky = __fsub_rn(pick(a4.x, a4.y, a4.z, ky), r.oy);
-    const float Akz = __fsub_rn(pick(a4.x, a4.y, a4.z, kz), r.oz);
-    const float Bkx = __fsub_rn(pick(b4.x, b4.y, b4.z, kx), r.ox);
-    const float Bky = __fsub_rn(pick(b4.x, b4.y, b4.z, ky), r.oy);
-    const float Bkz = __fsub_rn(pick(b4.x, b4.y, b4.z, kz), r.oz);
-    const float Ckx = __fsub_rn(pick(c4.x, c4.y, c4.z, kx), r.ox);
-    const float Cky = __fsub_rn(pick(c4.x, c4.y, c4.z, ky), r.oy);
-    const float Ckz = __fsub_rn(pick(c4.x, c4.y, c4.z, kz), r.oz);
-#endif
     const float Ax = __fsub_rn(Akx, __fmul_rn(r.Sx, Akz));
     const float Ay = __fsub_rn(Aky, __fmul_rn(r.Sy, Akz));
     const float Bx = __fsub_rn(Bkx, __fmul_rn(r.Sx, Bkz));
@@ -236,15 +218,9 @@ GBPT_DI bool intersect_tri(const RayPre& p, const RayShear& r, float4 a4, float4
     const float t = __fdiv_rn(T, det);
     if (!(t >= tmin && t <= tmax)) return false;
     t_out = t;
-#if GBPT_DEFER_UV
     u_out = V;
     v_out = W;
     det_out = det;
-#else
-    u_out = __fdiv_rn(V, det);
-    v_out = __fdiv_rn(W, det);
-    det_out = 1.0f;
-#endif
     return true;
 }
 
@@ -320,7 +296,7 @@ GBPT_DI float3 xform_vector(float4 r0, float4 r1, float4 r2, float3 v) {
 // 13 words, an odd stride: the lanes' words fall into different banks.
 struct LaneMem {
     RayShear ray;
-    float u, v, det; // GBPT_DEFER_UV: u, v are V, W of the test until divided by det
+    float u, v, det; // u, v are V, W of the test until divided by det
     uint32_t prim, geom, inst; // geom = kNoInst until a hit is found
     uint32_t pad;
 };
@@ -361,7 +337,6 @@ struct TraceState {
     GBPT_DI int sp() const { return (int)(pre.k >> 24); }
     GBPT_DI void push_sp() { pre.k += 1u << 24; }
     GBPT_DI void pop_sp() { pre.k -= 1u << 24; }
-    GBPT_DI void clear_sp() { pre.k &= 0x00FFFFFFu; }
 };
 
 // Where a launch's rays find their scene: in each ray's state (requests of several scenes share
@@ -393,7 +368,7 @@ GBPT_DI void set_ray(TraceState& s, const Scene& scene, float3 o, float3 d) {
     s.pre = ray_pre(o, d, s.lane->ray);
     s.pre.k |= ((7u - oct) << 8) | kept;
     const SceneRef& ref = scene.of(s);
-    s.tris = kTriCopies > 1 ? ref.tris + (size_t)s.pre.kz() * ref.tri_stride : ref.tris;
+    s.tris = ref.tris + (size_t)s.pre.kz() * ref.tri_stride;
 }
 
 // A span's start with -0 for +0, as intersect_node needs it. (The distance made +0 there instead
@@ -696,13 +671,9 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
             if (t < s.t || geom < s.lane->geom ||
                 (geom == s.lane->geom &&
                  (prim < s.lane->prim || (prim == s.lane->prim && s.inst < s.lane->inst)))) {
-#if GBPT_DEFER_UV
                 if ((tfl & kTriAlpha) && alpha(geom, prim, __fdiv_rn(u, det), __fdiv_rn(v, det)))
                     continue;
                 s.lane->det = det;
-#else
-                if ((tfl & kTriAlpha) && alpha(geom, prim, u, v)) continue;
-#endif
                 s.t = t;
                 s.lane->u = u;
                 s.lane->v = v;

@@ -12,15 +12,11 @@ namespace gbpt {
 
 struct DevScene; // device_scene.cuh
 
-// GBPT_TRI_AXIS_COPIES: each traversal triangle record is stored three times, its vertices'
-// coordinates permuted for each dominant ray axis kz to (kz + 1, kz + 2, kz) mod 3, so the
-// watertight test reads the ray's frame from memory instead of selecting 9 coordinates at run
-// time. Copy c of record i is record c n + i of the uploaded array (n records), so a ray reads
-// one contiguous copy. 0: one copy, coordinates selected at run time.
-#ifndef GBPT_TRI_AXIS_COPIES
-#define GBPT_TRI_AXIS_COPIES 1
-#endif
-constexpr int kTriCopies = GBPT_TRI_AXIS_COPIES ? 3 : 1;
+// Each traversal triangle record is stored three times, its vertices' coordinates permuted for each
+// dominant ray axis kz to (kz + 1, kz + 2, kz) mod 3, so the watertight test reads the ray's frame
+// from memory instead of selecting 9 coordinates at run time. Copy c of record i is record c n + i
+// of the uploaded array (n records), so a ray reads one contiguous copy.
+constexpr int kTriCopies = 3;
 
 // GBPT_ENV_ALIAS: next-event estimation picks the environment texel by alias tables (a row, then
 // a column: two dependent loads) instead of inverting the marginal and conditional CDFs (a

@@ -14,19 +14,24 @@ from conftest import ROOT
 from oracle import binding as O
 
 
-@pytest.fixture(scope="module")
-def host(native, tmp_path_factory):
+def _build(tmp, defines=()):
     from merian_gb300 import build as B
-    lib = tmp_path_factory.mktemp("traversal") / "libtraversal.so"
+    lib = tmp / "libtraversal.so"
     subprocess.run(["g++", "-O1", "-std=c++17", "-ftrivial-auto-var-init=pattern",
-                    "-ffp-contract=off", "-fPIC", "-shared", "-I", str(B.INCLUDE), "-I",
-                    str(B.CSRC), "-I", str(B._cuda_home() / "include"),
-                    str(ROOT / "tests" / "traversal_host.cpp"), "-o", str(lib)], check=True)
+                    "-ffp-contract=off", "-fPIC", "-shared", *[f"-D{d}" for d in defines],
+                    "-I", str(B.INCLUDE), "-I", str(B.CSRC), "-I",
+                    str(B._cuda_home() / "include"), str(ROOT / "tests" / "traversal_host.cpp"),
+                    "-o", str(lib)], check=True)
     fn = C.CDLL(str(lib)).traversal_host
     fn.restype = C.c_int64
     vp, u32, u64, i32 = C.c_void_p, C.c_uint32, C.c_uint64, C.c_int
     fn.argtypes = [vp, u64, vp, u64, vp, u64, i32, i32, vp, vp, u32, u32, u32, vp]
     return fn
+
+
+@pytest.fixture(scope="module")
+def host(native, tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("traversal"))
 
 
 def _soup():
@@ -113,6 +118,14 @@ def test_helpers_have_the_state_they_use(host, kind, mode, n, grid):
         assert np.array_equal(h[f][c].view(np.uint32), o[f][c].view(np.uint32)), f
     if kind == "instanced":
         assert np.array_equal(h["instance_id"][c], o["instance_index"][c])
+
+
+def test_former_build_options(native, tmp_path):
+    """A build that still sets the options of the deferred division and of the triangle records'
+    axis copies, which the traversal now always has, finds the same hits."""
+    fn = _build(tmp_path, ("GBPT_DEFER_UV=0", "GBPT_TRI_AXIS_COPIES=0"))
+    test_helpers_have_the_state_they_use(fn, "single", "query", 40, 4)
+    test_helpers_have_the_state_they_use(fn, "instanced", "tick of many scenes", 40, 4)
 
 
 def _sheets():
