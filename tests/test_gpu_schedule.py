@@ -273,3 +273,38 @@ def test_long_and_short_ticks(gpu_ctx, kind, height):
     finally:
         gpu_ctx.set_tuning()
         gpu_ctx.destroy_scene(sid)
+
+
+def test_sorted_few_pixels_of_many_samples(gpu_ctx):
+    """A pixel's sort key serves all its samples: requests of few pixels and many samples, around
+    the sizes of the sort's tiles and several to a tick, give the bits of unsorted shading, and
+    the primary pass does not grow with the samples of a pixel (its time with the sample sums is
+    that of unsorted shading; a factor of 2 covers the timer)."""
+    from merian_gb300 import scene as S
+    sid = gpu_ctx.upload(S.soup(n_triangles=20_000, n_geometries=64, env_size=(64, 32)))
+    cam = S.look_at((0.5, 0.5, -0.6), (0.5, 0.5, 0.5), (0.0, 1.0, 0.0), 45.0, 1.0)
+    jobs, keep = [], []
+    for px, spp in [(1, 1), (1, 2047), (3, 2049), (5, 4096), (37, 33), (2, 70_001)]:
+        pix = np.random.default_rng(px).choice(64 * 64, px, replace=False).astype(np.uint32)
+        p, k = S.render_params(64, 64, spp, 4, nee=True, rr_depth=3, frame=spp, pixels=pix)
+        jobs.append((sid, cam, p))
+        keep.append((pix, k))
+    pix = np.arange(64, dtype=np.uint32) * 61
+    many, k = S.render_params(64, 64, 1 << 16, 2, nee=False, frame=1, pixels=pix)
+    try:
+        outs, other = [], []
+        for sort in (0, 1, -1):
+            gpu_ctx.set_tuning(sort_materials=sort)
+            outs.append([gpu_ctx.render(*j) for j in jobs] + gpu_ctx.render_batch(jobs))
+            gpu_ctx.set_profiling(1)
+            other.append(min(gpu_ctx.render(sid, cam, many, stats=True)[1].other_ms
+                             for _ in range(3)))
+            gpu_ctx.set_profiling(0)
+        for o in outs[1:]:
+            assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32))
+                       for a, b in zip(outs[0], o))
+        assert max(other[1:]) < 2 * other[0], other
+    finally:
+        gpu_ctx.set_profiling(0)
+        gpu_ctx.set_tuning()
+        gpu_ctx.destroy_scene(sid)
