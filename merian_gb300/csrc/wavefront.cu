@@ -647,6 +647,9 @@ __global__ void __launch_bounds__(256) k_sort_scatter(TickArgs t, int k, uint32_
 // Bound by memory (32 B per sample, 16 B per pixel), and at few samples by the lanes without one:
 // a warp per pixel, 31 of 32 lanes idle at 1 sample per pixel, made a batch of 48 small requests
 // 35.2 instead of 32.9 ms and 8 accumulated 960x540 frames 42.3 instead of 41.6 ms.
+// At many samples the loads' latency binds: eight are in flight per lane, added in order (one pixel
+// of 2^20 samples 3.5 ms; one at a time 10.3, in a warp of constant stride that the compiler unrolled
+// by four 7.7).
 __global__ void __launch_bounds__(128) k_finalize(TickArgs t) {
     wait_for_predecessor();
     const uint32_t G = t.hdr->sum_lanes;
@@ -669,8 +672,7 @@ __global__ void __launch_bounds__(128) k_finalize(TickArgs t) {
             ay = pc[4].w;
             az = pc[5].w;
         }
-        for (uint32_t s = lane; s < S; s += G) {
-            float4 v = t.w.path[2 * (base + s) + 1];
+        auto add = [&](float4 v) {
             if (demod) {
                 v.x = v.x / ax;
                 v.y = v.y / ay;
@@ -680,10 +682,22 @@ __global__ void __launch_bounds__(128) k_finalize(TickArgs t) {
                 cr += v.x;
                 cg += v.y;
                 cb += v.z;
-                const float l = yuv_luminance(f3(v.x, v.y, v.z));
-                m += l * l;
+                // yuv_luminance, its rounding fixed: the two loops give the same bits
+                const float l = __fmaf_rn(
+                    v.z, 0.114f, __fmaf_rn(v.y, 0.587f, __fmul_rn(v.x, 0.299f)));
+                m = __fmaf_rn(l, l, m);
             }
+        };
+        const float4* radiance = t.w.path + 2 * base + 1;
+        uint32_t s = lane;
+        for (; s + 7u * G < S; s += 8u * G) {
+            float4 v[8];
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) v[j] = radiance[2 * (uint64_t)(s + j * G)];
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j) add(v[j]);
         }
+        for (; s < S; s += G) add(radiance[2 * (uint64_t)s]);
         for (uint32_t off = G >> 1; off > 0; off >>= 1) {
             cr += __shfl_xor_sync(0xFFFFFFFFu, cr, off);
             cg += __shfl_xor_sync(0xFFFFFFFFu, cg, off);

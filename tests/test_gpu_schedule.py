@@ -308,3 +308,57 @@ def test_sorted_few_pixels_of_many_samples(gpu_ctx):
         gpu_ctx.set_profiling(0)
         gpu_ctx.set_tuning()
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("spp", [1, 8, 33, 7 * 32, 8 * 32 - 1, 8 * 32, 8 * 32 + 1, 9 * 32 - 1,
+                                 16 * 32 + 5])
+def test_sample_sum_of_equal_samples(gpu_ctx, spp):
+    """The samples of a pixel that sees the environment are equal: their sum is NumPy's in the
+    kernel's order (each lane its samples one after the other, several loads in flight or not,
+    then the tree), to the last bit."""
+    import test_gpu_errors as E
+    from merian_gb300 import scene as S
+    sc = E.quad()
+    sc.env = np.tile(np.array([0.1, 0.7, 0.3, 1.0], np.float32), (8, 16, 1))
+    sid = gpu_ctx.upload(sc)
+    cam = S.look_at((0, 0, 0), (0, 0, -1), (0, 1, 0), 60.0, 1.0)
+    try:
+        p, _ = S.render_params(3, 3, 1, 1, frame=2)
+        v = gpu_ctx.render(sid, cam, p)[:, :3]
+        p, _ = S.render_params(3, 3, spp, 1, frame=2)
+        out = gpu_ctx.render(sid, cam, p)
+    finally:
+        gpu_ctx.destroy_scene(sid)
+    fma = lambda a, b, c: np.float32(np.longdouble(a) * np.longdouble(b) + np.longdouble(c))
+    group = 1
+    while group < min(spp, 32):
+        group *= 2
+    for px in range(9):
+        r, g, b = v[px]
+        lum = fma(b, np.float32(0.114), fma(g, np.float32(0.587), np.float32(0.299) * r))
+        lanes = np.zeros((group, 4), np.float32)
+        for lane in range(group):
+            for _ in range(lane, spp, group):
+                lanes[lane, :3] += v[px]
+                lanes[lane, 3] = fma(lum, lum, lanes[lane, 3])
+        off = group // 2
+        while off:
+            lanes = lanes + lanes[np.arange(group) ^ off]
+            off //= 2
+        want = lanes[0] * (np.float32(1.0) / np.float32(spp))
+        assert np.array_equal(out[px].view(np.uint32), want.view(np.uint32)), px
+
+
+def test_sample_sum_of_one_pixel(gpu_ctx, room):
+    """2^20 samples of a pixel with the primary pass in 5 ms: with one load after the other in
+    flight their sum takes more than twice that, with eight 2.7 ms."""
+    from merian_gb300 import scene as S
+    sid, cam = room
+    pix = np.array([64 * 30 + 31], np.uint32)
+    p, k = S.render_params(64, 64, 1 << 20, 2, frame=4, pixels=pix)
+    try:
+        gpu_ctx.set_profiling(1)
+        ms = min(gpu_ctx.render(sid, cam, p, stats=True)[1].other_ms for _ in range(3))
+    finally:
+        gpu_ctx.set_profiling(0)
+    assert ms < 5
