@@ -374,9 +374,12 @@ GBPT_API int gbpt_get_tuning(gbpt_ctx* ctx, gbpt_tuning* tuning);
  * (2^24 .. 2^21 paths, largest first; a smaller tick must be at least 2 % faster to be kept, since
  * larger ticks let more requests share one) with material sorting off and on (8 candidates,
  * ms_out in ascending tick size); then, from the best so far,
- * one parameter at a time: trace_refill_lanes in {12, 16, 20, 24, 28} (5), trace_postpone_lanes in
- * {2, 4, 6, 8, 12} (5), trace_blocks_per_sm in {6, 7, all resident} (3). ms_out, when non-NULL,
- * receives GBPT_AUTOTUNE_CANDIDATES times in that order (NaN for candidates not run). Results are
+ * one parameter at a time: trace_refill_lanes in {12, 16, 20, 24, 28} (5), trace_postpone_lanes (5
+ * times, each the best so far: without effect, it stays at its default and nothing is rendered),
+ * trace_blocks_per_sm in {6, 7, all resident} (3). The sorting it returns is 0 or 1, for every
+ * vertex and request of the context; a caller whose other requests are smaller can set
+ * sort_materials back to -1. ms_out, when non-NULL, receives GBPT_AUTOTUNE_CANDIDATES times in
+ * that order (NaN for candidates not run). Results are
  * cached per (scene size, frame size, path length, estimator) bucket: a repeated call for the same
  * bucket applies the cached tuning without rendering. Outputs are discarded. */
 #define GBPT_AUTOTUNE_CANDIDATES 32

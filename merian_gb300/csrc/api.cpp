@@ -1334,10 +1334,10 @@ GBPT_API int gbpt_get_tuning(gbpt_ctx* ctx, gbpt_tuning* t) {
 // The autotuner: candidate tunings rendered on one representative request, the fastest kept.
 // Outputs do not depend on the tuning (tick size, shading order and warp scheduling only change
 // the schedule), so only time is compared. Stage 1 crosses tick size and material sorting; the
-// traversal's refill threshold, the postponement threshold (now without effect: its candidates tie)
-// and its blocks per SM are then searched one at a
-// time from the best so far. Results are cached per bucket of scene size, frame size, path length
-// and estimator.
+// traversal's refill threshold and its blocks per SM are then searched one at a time from the best
+// so far. trace_postpone_lanes has no effect: its candidates are not rendered, its result is the
+// default and their times are the best time so far. Results are cached per bucket of scene size,
+// frame size, path length and estimator.
 GBPT_API int gbpt_autotune(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* camera,
                            const gbpt_render_params* p, gbpt_tuning* out, double* ms_out) {
     int rc = check_ctx(ctx);
@@ -1460,7 +1460,7 @@ GBPT_API int gbpt_autotune(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam
             }
         }
     }
-    const int refill[5] = {12, 16, 20, 24, 28}, postpone[5] = {2, 4, 6, 8, 12};
+    const int refill[5] = {12, 16, 20, 24, 28};
     const int blocks[3] = {6, 7, 0};
     const gbpt_tuning stage1 = best;
     for (int k = 0; k < 5; ++k) {
@@ -1468,15 +1468,10 @@ GBPT_API int gbpt_autotune(gbpt_ctx* ctx, uint32_t scene, const gbpt_camera* cam
         t.trace_refill_lanes = refill[k];
         if ((rc = consider(t, 8 + k))) return rc;
     }
+    for (int k = 0; k < 5; ++k) ms_all[13 + k] = best_ms;
     const gbpt_tuning stage2 = best;
-    for (int k = 0; k < 5; ++k) {
-        gbpt_tuning t = stage2;
-        t.trace_postpone_lanes = postpone[k];
-        if ((rc = consider(t, 13 + k))) return rc;
-    }
-    const gbpt_tuning stage3 = best;
     for (int k = 0; k < 3; ++k) {
-        gbpt_tuning t = stage3;
+        gbpt_tuning t = stage2;
         t.trace_blocks_per_sm = blocks[k];
         if ((rc = consider(t, 18 + k))) return rc;
     }

@@ -362,3 +362,19 @@ def test_sample_sum_of_one_pixel(gpu_ctx, room):
     finally:
         gpu_ctx.set_profiling(0)
     assert ms < 5
+
+
+def test_autotuner_leaves_out_the_postponement(gpu_ctx):
+    """trace_postpone_lanes has no effect: the autotuner renders none of its five values, answers
+    the default and gives the best time so far for them."""
+    from merian_gb300 import scene as S
+    sid = gpu_ctx.upload(S.soup(n_triangles=3_000, n_geometries=8, env_size=(32, 16)))
+    cam = S.look_at((0.5, 0.5, -0.6), (0.5, 0.5, 0.5), (0.0, 1.0, 0.0), 45.0, 1.0)
+    p, _ = S.render_params(96, 96, 3, 7, nee=True, rr_depth=2, frame=1)
+    try:
+        t, ms = gpu_ctx.autotune(sid, cam, p)
+        assert len(ms) == 21 and t.trace_postpone_lanes == 6
+        assert ms[13:18] == [ms[13]] * 5 and ms[13] in ms[:13]
+    finally:
+        gpu_ctx.set_tuning()
+        gpu_ctx.destroy_scene(sid)
