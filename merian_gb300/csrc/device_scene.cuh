@@ -296,7 +296,9 @@ GBPT_DI float3 xform_vector(float4 r0, float4 r1, float4 r2, float3 v) {
 // 13 words, an odd stride: the lanes' words fall into different banks.
 struct LaneMem {
     RayShear ray;
-    float u, v, det; // u, v are V, W of the test until divided by det
+    // u, v are V, W of the test until divided by det. kSignedZero: det has the sign of the hit's t
+    // (all three may be negated, which leaves the quotients as they are)
+    float u, v, det;
     uint32_t prim, geom, inst; // geom = kNoInst until a hit is found
     uint32_t pad;
 };
@@ -371,9 +373,18 @@ GBPT_DI void set_ray(TraceState& s, const Scene& scene, float3 o, float3 d) {
     s.tris = ref.tris + (size_t)s.pre.kz() * ref.tri_stride;
 }
 
-// A span's start with -0 for +0, as intersect_node needs it. (The distance made +0 there instead
-// cost a register: a million closest hits 640 against 626 us.)
+// A span's start with -0 for +0 and its end with +0 for -0, as intersect_node needs them. (Made +0
+// in the box test instead, the end cost a register there: a million closest hits 640 against 626
+// us.)
 GBPT_DI float span_start(float tmin) { return tmin == 0.0f ? -0.0f : tmin; }
+GBPT_DI float span_end(float tmax) { return __fadd_rn(tmax, 0.0f); }
+
+// Whether a hit at -0 leaves a span that ends at +0, its sign kept in LaneMem::det: wherever a
+// direction can be infinite, the caller's or one transformed into an instance. The bounce and
+// shadow rays of single-level scenes are normalised; there the different registers of the
+// acceptance cost 37,003 listed pixels 1.60 instead of 1.54 ms.
+template <TraceMode MODE, bool TWO_LEVEL>
+constexpr bool kSignedZero = MODE != kTraceMixed || TWO_LEVEL;
 
 template <class Scene>
 GBPT_DI void trace_init(TraceState& s, const Scene& scene, float3 o, float3 d, float tmin,
@@ -386,7 +397,7 @@ GBPT_DI void trace_init(TraceState& s, const Scene& scene, float3 o, float3 d, f
     s.ngroup = make_uint2(0u, 0x80000000u);
     s.tgroup = make_uint2(0u, 0u);
     s.tmin = span_start(tmin);
-    s.t = tmax;
+    s.t = span_end(tmax);
     s.lane->u = s.lane->v = 0.0f;
     s.lane->prim = s.lane->geom = s.lane->inst = kNoInst;
     s.inst = kNoInst;
@@ -522,10 +533,11 @@ GBPT_DI void intersect_node(const TraceState& s, const uint4* nodes, uint32_t ni
     const bool negz = (oct_inv & 4u) == 0u;
     // the children missed, the first child in the highest bit: the sign of cmax - cmin is set
     // when cmin <= cmax is false. Neither is NaN (trace_init ends such rays), and inf - inf is the
-    // canonical, positive NaN. It is also set for cmin = +0 and cmax = -0, the distance of a hit
-    // at the origin along a negative axis (-0 - +0 = -0): so a span never starts at +0
-    // (span_start), and a near plane, which the slack puts before the box, is +0 only where the
-    // box begins beyond 0.
+    // canonical, positive NaN. It is also set for cmin = +0 and cmax = -0, though 0 <= -0
+    // (-0 - +0 = -0), which must not meet: cmax is -0 only as the distance, after a hit at the
+    // origin along a negative axis (span_end, kSignedZero), cmin is +0 only as a near plane
+    // (span_start), and that where the box begins beyond 0, since the slack puts it before the
+    // box - except along an infinite direction, whose planes are all 0.
     uint32_t miss = 0;
     auto add = [&](float cmin, float cmax) {
         miss = __funnelshift_l(__float_as_uint(__fsub_rn(cmax, cmin)), miss, 1);
@@ -673,6 +685,14 @@ GBPT_DI bool trace_loop(TraceState& s, const Scene& scene, StackRef&& st, const 
                  (prim < s.lane->prim || (prim == s.lane->prim && s.inst < s.lane->inst)))) {
                 if ((tfl & kTriAlpha) && alpha(geom, prim, __fdiv_rn(u, det), __fdiv_rn(v, det)))
                     continue;
+                if (kSignedZero<MODE, TWO_LEVEL>) {
+                    const uint32_t neg =
+                        (__float_as_uint(t) ^ __float_as_uint(det)) & 0x80000000u;
+                    det = __uint_as_float(__float_as_uint(det) ^ neg);
+                    u = __uint_as_float(__float_as_uint(u) ^ neg);
+                    v = __uint_as_float(__float_as_uint(v) ^ neg);
+                    t = span_end(t);
+                }
                 s.lane->det = det;
                 s.t = t;
                 s.lane->u = u;
@@ -860,6 +880,7 @@ __device__ __forceinline__ void trace_persistent(const Scene& scene, uint32_t n,
     auto store = [&](uint32_t i, TraceState& s) {
         Hit h{s.t, s.lane->u, s.lane->v, s.lane->prim, s.lane->geom, s.lane->inst};
         if (h.geom != kNoInst) {
+            if (kSignedZero<MODE, TWO_LEVEL> && h.t == 0.0f) h.t = copysignf(0.0f, s.lane->det);
             h.u = __fdiv_rn(h.u, s.lane->det);
             h.v = __fdiv_rn(h.v, s.lane->det);
         }

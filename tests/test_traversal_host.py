@@ -228,6 +228,89 @@ def test_hits_at_the_origin(host, kind, mode, grid):
         assert np.array_equal(w["t"].view(np.uint32), h["t"].view(np.uint32))
 
 
+def _special_rays(n):
+    """Rays with NaN, infinite, zero and denormal components of origin and direction among
+    ordinary ones, and spans with such ends."""
+    from merian_gb300 import _native as N
+    rng = np.random.default_rng(n)
+    rays = np.zeros(n, N.RAY_DTYPE)
+    rays["origin"] = rng.uniform(-0.1, 1.1, (n, 3))
+    rays["direction"] = rng.normal(size=(n, 3))
+    rays["tmax"] = 1e7
+    odd = np.array([np.nan, np.inf, -np.inf, 0.0, -0.0, 1e-40, -1e-40, 1e-30, 3e38], np.float32)
+    for f in ("origin", "direction"):
+        k = rng.uniform(size=(n, 3)) < 0.12
+        rays[f][k] = rng.choice(odd, k.sum())
+    for f in ("tmin", "tmax"):
+        k = rng.uniform(size=n) < 0.1
+        rays[f][k] = rng.choice(odd, k.sum())
+    return rays
+
+
+def _infinite_rays(n):
+    """Rays along an infinite direction: t is +0 or -0 for every triangle they meet, and the planes
+    of the boxes have no slack."""
+    from merian_gb300 import _native as N
+    rng = np.random.default_rng(n + 1)
+    rays = np.zeros(n, N.RAY_DTYPE)
+    rays["origin"] = rng.uniform(0, 1, (n, 3))
+    rays["direction"] = rng.normal(size=(n, 3))
+    rays["direction"][np.arange(n), rng.integers(0, 3, n)] = rng.choice([-np.inf, np.inf], n)
+    rays["tmin"] = rng.choice(np.array([0.0, -0.0, -1.0], np.float32), n)
+    rays["tmax"] = rng.choice(np.array([1e7, 0.0, -0.0], np.float32), n)
+    return rays
+
+
+def _same_as_walk(h, w, any_hit):
+    miss = w["geometry_index"] == 0xFFFFFFFF
+    assert miss.any() and not miss.all()
+    assert np.array_equal(h["geometry_index"] == 0xFFFFFFFF, miss)
+    if not any_hit:
+        for f in ("t", "primitive_id", "geometry_index", "barycentrics"):
+            assert np.array_equal(h[f][~miss].view(np.uint32), w[f][~miss].view(np.uint32)), f
+
+
+@pytest.mark.parametrize("make", [_special_rays, _infinite_rays])
+@pytest.mark.parametrize("grid", [64, 3])
+def test_special_values(host, make, grid):
+    """The hits of the walk that visits one ray at a time, which compares the boxes' distances
+    where the traversal takes signs of differences."""
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    nodes, tris, _ = S.build_bvh(_soup(), N.BVH_MEDIUM)
+    rays = make(600)
+    h, bad = _run(host, nodes, tris, None, rays, np.zeros(len(rays)), False, 0, grid)
+    assert bad == 0
+    w, _ = O.cwbvh_trace(nodes, tris, rays, hit_dtype=N.HIT_DTYPE)
+    _same_as_walk(h, w, False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [_special_rays, _infinite_rays])
+@pytest.mark.parametrize("any_hit", [False, True], ids=["closest", "any"])
+def test_gpu_special_values(gpu_ctx, make, any_hit):
+    import torch
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    sc = _soup()
+    nodes, tris, _ = S.build_bvh(sc)
+    sid = gpu_ctx.upload(sc)
+    try:
+        for n in (200, 20_000):
+            rays = make(n)
+            w, _ = O.cwbvh_trace(nodes, tris, rays, any_hit=any_hit, hit_dtype=N.HIT_DTYPE)
+            r = torch.from_numpy(rays.view(np.float32).reshape(n, 8)).cuda()
+            h = torch.zeros((n, 8), dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            for counted in (False, True):
+                gpu_ctx.trace(sid, r.data_ptr(), n, h.data_ptr(), any_hit=any_hit,
+                              counted=counted)
+                gpu_ctx.synchronize()
+                _same_as_walk(np.frombuffer(h.cpu().numpy().tobytes(), N.HIT_DTYPE), w, any_hit)
+    finally:
+        gpu_ctx.destroy_scene(sid)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["single", "instanced"])
 def test_gpu_hits_at_the_origin(gpu_ctx, kind):

@@ -2,8 +2,8 @@
 // of a warp run as coroutines that meet at every warp-wide operation, blocks of one warp run one
 // after the other. Reads through __ldg are checked against the scene's arrays (counted and
 // answered with zeros when outside), and -ftrivial-auto-var-init=pattern fills what the code
-// leaves unset, so a use of unset lane state shows as a wrong hit or a counted read. NaNs of
-// subtractions are the GPU's (0x7fffffff).
+// leaves unset, so a use of unset lane state shows as a wrong hit or a counted read. NaNs and the
+// order of signed zeros are the GPU's.
 #include <ucontext.h>
 
 #include <cmath>
@@ -175,6 +175,19 @@ inline uint32_t atomicOr(uint32_t* p, uint32_t v) {
     return old;
 }
 using std::min;
+// the GPU's: a NaN gives way to a number, -0 is less than +0
+namespace gbpt {
+inline float fmaxf(float a, float b) {
+    if (a != a) return b;
+    if (b != b) return a;
+    return a > b || (a == b && !std::signbit(a)) ? a : b;
+}
+inline float fminf(float a, float b) {
+    if (a != a) return b;
+    if (b != b) return a;
+    return a < b || (a == b && std::signbit(a)) ? a : b;
+}
+} // namespace gbpt
 
 #define GBPT_BOX_FMA2 0 // the pairs round each plane as the single ones do
 #include "device_scene.cuh"
