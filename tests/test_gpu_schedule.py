@@ -364,6 +364,33 @@ def test_sample_sum_of_one_pixel(gpu_ctx, room):
     assert ms < 5
 
 
+@pytest.mark.parametrize("touched", ["none", "first half", "every other page", "all"])
+def test_host_outputs_in_any_pages(gpu_ctx, room, touched):
+    """Host outputs whose pages are absent, partly or wholly present, at the end of a mapping and
+    not at a page's start: the image, and nothing beside it."""
+    import ctypes as C
+    import mmap
+    from merian_gb300 import _native as N
+    from merian_gb300 import scene as S
+    sid, cam = room
+    w = h = 160  # 400 KB
+    p, _ = S.render_params(w, h, 1, 2, frame=9)
+    ref = gpu_ctx.render(sid, cam, p)
+    size = -(-(ref.nbytes + 4096) // mmap.PAGESIZE) * mmap.PAGESIZE
+    with mmap.mmap(-1, size) as m:
+        buf = np.frombuffer(m, np.uint8)
+        at = size - ref.nbytes
+        if touched != "none":
+            step = mmap.PAGESIZE * (2 if touched == "every other page" else 1)
+            buf[:size // 2 if touched == "first half" else size:step] = 7
+        before = buf[:at].copy() if touched != "none" else np.zeros(at, np.uint8)
+        out = C.c_void_p(buf.ctypes.data + at)
+        N.check(gpu_ctx.lib.gbpt_render(gpu_ctx.handle, sid, C.byref(cam), C.byref(p), out, None))
+        assert np.array_equal(buf[at:], ref.view(np.uint8).reshape(-1))
+        assert np.array_equal(buf[:at], before)
+        del buf
+
+
 def test_autotuner_leaves_out_the_postponement(gpu_ctx):
     """trace_postpone_lanes has no effect: the autotuner renders none of its five values, answers
     the default and gives the best time so far for them."""
@@ -378,3 +405,37 @@ def test_autotuner_leaves_out_the_postponement(gpu_ctx):
     finally:
         gpu_ctx.set_tuning()
         gpu_ctx.destroy_scene(sid)
+
+
+@pytest.mark.parametrize("differs", ["nothing", "position", "jitter", "far plane", "scene"])
+def test_graph_gbuffer_of_another_view(gpu_ctx, tmp_path, differs):
+    """A renderer takes primary hits from its G-buffer only when that was traced for the same
+    scene and camera: here the G-buffer's come from a scene file, the renderer's from the graph's
+    call. Always the frame of the renderer's own view."""
+    from test_gltf import build_scene
+    from merian_gb300 import node
+    from merian_gb300 import scene as S
+    path, _ = build_scene(tmp_path, "glb")
+    sc, cam, _, _ = S.load_gltf(path)
+    w, h = 72, 48
+    other = gpu_ctx.upload(sc)  # the file's scene gets the next id
+    if differs == "position":
+        cam.position[0] += 0.125
+    elif differs == "jitter":
+        cam.jitter[0] = 0.375
+    elif differs == "far plane":
+        cam.far_plane = 2.0
+    try:
+        with node.Graph(gpu_ctx, {"nodes": {
+                "s": {"type": "GLTF Scene", "properties": {"file": str(path)},
+                      "outputs": ["scene->g.scene"]},
+                "g": {"type": "GBuffer (Raytraced)", "properties": {"width": w, "height": h},
+                      "outputs": ["gbuffer->r.gbuffer"]},
+                "r": {"type": "Render (Path-traced)", "properties": {"samples per pixel": 2}}}}) as g:
+            g.run(other if differs == "scene" else other + 1, cam, (w, h), 2)
+            out = g.output("r.irradiance").reshape(-1, 4)
+        p, _ = S.render_params(w, h, 2, 5, frame=1)
+        ref = gpu_ctx.render(other, cam, p)
+        assert np.array_equal(out.view(np.uint32), ref.view(np.uint32))
+    finally:
+        gpu_ctx.destroy_scene(other)
