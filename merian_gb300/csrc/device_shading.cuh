@@ -425,9 +425,9 @@ template <class K> int persistent_grid(K kernel) {
 #define GBPT_TRACE_BLOCKS_PER_SM 8
 #endif
 constexpr int kTraceBlocksPerSM = GBPT_TRACE_BLOCKS_PER_SM;
-// 9 in long queues of single-level scenes, where the ninth block hides more of the others' waiting
+// 9 in long ticks (kLongTick) of single-level scenes, where the ninth block hides more of the others' waiting
 // than its spills cost (1080p soup frame 235.0 instead of 239.8 ms, 640x360 7.65 instead of 7.80; a
-// tenth costs more: 227.7 instead of 226.1); short queues end with a few rays whose latency the
+// tenth costs more: 227.7 instead of 226.1); short ticks end with a few rays whose latency the
 // spills add to (37,003 pixels x 8 1.58 instead of 1.50). The two-level variants hold the instance
 // as well and spilled at 8 blocks until the world ray moved to shared memory; now 8 beat 7
 // (instanced 1280x720 frame 3.56 instead of 3.62 ms, its G-buffer 0.757 instead of 0.766).

@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(128, kShadeBlocksPerSM)
 // are added to their path (one shadow ray per path and vertex, so no two lanes write the same
 // path; the closest hits touch no path). `parts`: 1 the closest hits, 2 the shadow rays, 3 both in
 // one launch, the longer traversals first.
-// Bound by issue slots (65 % active, 15 of 32 lanes) while the pool lasts, then by the latency of
+// Bound by issue slots (69 % active, 15 of 32 lanes) while the pool lasts, then by the latency of
 // the last rays: one launch has one such tail where a launch for each kind had two (a 64x64 frame
 // 0.28 instead of 0.41 ms, the instanced 1280x720 frame of path length 16 5.6 instead of 7.6, the
 // 640x360 soup frame 8.6 instead of 9.4; the clears of the counters, now one per tick instead of
@@ -942,7 +942,8 @@ Grids launch_grids() {
 // variants without a feature leave its code out; they find the same hits on scenes without it).
 // Ticks of at least this many paths trace with 9 blocks per SM (trace_blocks): between the 0.3 M
 // paths that lose by it and the 3.7 M that gain; at 1 M (256x256 room, 16 samples) both take
-// 1.02 ms.
+// 1.02 ms. It is a rule of the tick: all its vertices take the variant, also the late ones, whose
+// queues are short (measured as whole frames only).
 constexpr uint32_t kLongTick = 1u << 20;
 
 // A kernel that begins with wait_for_predecessor().

@@ -931,8 +931,7 @@ ORACLE_API int oracle_trace_rays(void* sp, const gbpt_ray* rays, uint32_t n, uin
 
 // ---- a walk of the package's CWBVH (test infrastructure) -------------------------------------
 // A host restatement of the device traversal of one ray (merian_gb300/csrc/device_scene.cuh:
-// set_ray, intersect_node, trace_loop in the per-thread order, i.e. without postponed triangle
-// groups) over the 80-byte nodes and 48-byte triangle records gbpt_bvh_build returns, for
+// set_ray, intersect_node, trace_loop, one ray at a time) over the 80-byte nodes and 48-byte triangle records gbpt_bvh_build returns, for
 // single-level trees. Every box-test operation is rounded once in the device's order
 // (__fmul_rn / __fsub_rn / __fmaf_rn there, -ffp-contract=off and std::fma here), so the walk
 // makes the same box decisions: it visits the same nodes and tests the same triangles as the
