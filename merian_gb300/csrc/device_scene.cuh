@@ -291,8 +291,9 @@ GBPT_DI float3 xform_vector(float4 r0, float4 r1, float4 r2, float3 v) {
 // accepted, two or three times a ray) and the triangle test's ray (read while the triangle's
 // record is on its way). In registers these words made the traversal spill others, 96 to 136 bytes
 // a thread at 8 and 9 blocks per SM, and what it spilled missed L1 two times in three; now it
-// spills 8 to 48, in ticks of several two-level scenes up to 114 (640x360 soup frame 7.18 instead of 7.35 ms, 1080p 226.1 instead of 227.4, 37,003
-// listed pixels 1.50 instead of 1.55, a million closest hits 0.645 instead of 0.652).
+// spills 8 to 48, in ticks of several two-level scenes up to 114 (640x360 soup frame 7.18 instead
+// of 7.35 ms, 1080p 226.1 instead of 227.4, 37,003 listed pixels 1.50 instead of 1.55, a million
+// closest hits 0.645 instead of 0.652).
 // 13 words, an odd stride: the lanes' words fall into different banks.
 struct LaneMem {
     RayShear ray;
